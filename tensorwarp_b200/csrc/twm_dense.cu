@@ -10,6 +10,7 @@
 #include "twm_dense_attn_tc.cuh"
 #include "twm_dense_common.cuh"
 #include "twm_dense_decode.cuh"
+#include "twm_dense_f32.cuh"
 #include "twm_dense_gla.cuh"
 #include "twm_dense_latent.cuh"
 #include "twm_dense_moe.cuh"
@@ -361,6 +362,51 @@ twm_status gemm_tc_any(const bf16* a, int lda, const bf16* w, int ldw, void* c, 
     return invalid("epilogue");
 }
 
+// The FP32 product on 16-byte copies.  Rows are spread evenly over tiles of up to 64; K over as many CTAs of a cluster as
+// cost least, counted in stages of 32 K: waves of two CTAs to an SM, and eight stages' time for the exchange of the sums.
+template <int TM, int EPI>
+twm_status gemm_f32_launch(const GemmF32Args& g, int n_tiles, int flags, void* stream)
+{
+    return launch("gemm_f32", gemm_f32_kernel<TM, EPI>, dim3((unsigned)((long)n_tiles * g.m_tiles * g.splits)), F32_THREADS, f32_smem_bytes(TM),
+                  flags, stream, g.splits > 1 ? g.splits : 0, g);
+}
+template <int EPI>
+twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, int ldc, int M, int N, int K, int flags, void* stream)
+{
+    int sms = 148;
+    TRY(device(&sms));
+    GemmF32Args g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, (M + 63) / 64, 1};
+    const int out = EPI == TWM_EPI_GELU_GLU ? F32_BN / 2 : F32_BN, n_tiles = (N + out - 1) / out, k_tiles = (K + F32_BK - 1) / F32_BK;
+    const int tm = ((M + g.m_tiles - 1) / g.m_tiles + 7) / 8;
+    long best = -1;
+    for (int s = 1; s <= F32_MAX_SPLITS; ++s) {
+        const long waves = ((long)n_tiles * g.m_tiles * s + 2 * sms - 1) / (2 * sms), cost = waves * ((k_tiles + s - 1) / s + (s > 1 ? 8 : 0));
+        if (best < 0 || cost < best) { best = cost; g.splits = s; }
+    }
+    switch (tm) {
+        case 1: return gemm_f32_launch<1, EPI>(g, n_tiles, flags, stream);
+        case 2: return gemm_f32_launch<2, EPI>(g, n_tiles, flags, stream);
+        case 3: return gemm_f32_launch<3, EPI>(g, n_tiles, flags, stream);
+        case 4: return gemm_f32_launch<4, EPI>(g, n_tiles, flags, stream);
+        case 5: return gemm_f32_launch<5, EPI>(g, n_tiles, flags, stream);
+        case 6: return gemm_f32_launch<6, EPI>(g, n_tiles, flags, stream);
+        case 7: return gemm_f32_launch<7, EPI>(g, n_tiles, flags, stream);
+        default: return gemm_f32_launch<8, EPI>(g, n_tiles, flags, stream);
+    }
+}
+// rows that start on 16-byte boundaries
+bool f32_fits(const float* a, int lda, const float* w, int ldw)
+{
+    return lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0;
+}
+bool f32_fits(const bf16*, int, const bf16*, int) { return false; }
+twm_status gemm_f32_any(const bf16*, int, const bf16*, int, void*, int, int, int, int, int, int, void*) { return invalid("the FP32 product takes float"); }
+twm_status gemm_f32_any(const float* a, int lda, const float* w, int ldw, void* c, int ldc, int M, int N, int K, int epi, int flags, void* stream)
+{
+    return epi == TWM_EPI_GELU_GLU ? gemm_f32<TWM_EPI_GELU_GLU>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream)
+                                   : gemm_f32<TWM_EPI_STORE_F32>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream);
+}
+
 template <typename T>
 twm_status gemm(const T* a, int lda, const T* w, int ldw, void* c, int ldc, int M, int N, int K, int epi, int kernel, int flags,
                 void* stream)
@@ -370,6 +416,8 @@ twm_status gemm(const T* a, int lda, const T* w, int ldw, void* c, int ldc, int 
     if (kernel >= 2 && !fits) return invalid("the tcgen05 product takes bfloat16 rows on 16-byte boundaries");
     if (kernel >= 2 || (kernel == 0 && fits))
         return gemm_tc_any(a, lda, w, ldw, c, ldc, M, N, K, epi, kernel > 2 ? kernel : 0, flags, stream);
+    if (f32_fits(a, lda, w, ldw) && (epi == TWM_EPI_STORE || epi == TWM_EPI_STORE_F32 || epi == TWM_EPI_GELU_GLU))
+        return gemm_f32_any(a, lda, w, ldw, c, ldc, M, N, K, epi, flags, stream);
     const dim3 grid((N + ST - 1) / ST, (M + ST - 1) / ST);
     switch (epi) {
         case TWM_EPI_STORE:

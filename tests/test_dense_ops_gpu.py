@@ -55,3 +55,25 @@ def test_gemm_rows_with_longer_strides_and_no_bleed():
         got = gemm(a[:70, :80], w[:66, :80], _dense.EPI_STORE_F32, kernel, 66)
         ref = a[:70, :80].double() @ w[:66, :80].double().T
         assert float((got - ref).abs().max()) < 1e-3
+
+
+@pytest.mark.parametrize("m,n,k,lda,ldw", [(1, 1, 1, 4, 4), (8, 127, 33, 36, 40), (9, 129, 2050, 2052, 2052), (64, 128, 32, 32, 32), (65, 1, 5000, 5000, 5000),
+                                           (130, 300, 96, 99, 96), (41, 70, 64, 64, 65)])
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
+def test_gemm_f32_edges(m, n, k, lda, ldw, epi):
+    """FP32 tiles around their edges, K shared by a cluster and not, K that ends inside 16 bytes, and rows off 16-byte boundaries."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rows = 2 * n if epi == _dense.EPI_GELU_GLU else n
+    a = torch.full((m, lda), 1e30, device="cuda")
+    w = torch.full((rows, ldw), 1e30, device="cuda")
+    a[:, :k] = torch.randn((m, k), generator=gen, device="cuda")
+    w[:, :k] = torch.randn((rows, k), generator=gen, device="cuda") / math.sqrt(k)
+    got = gemm(a[:, :k], w[:, :k], epi, 0, n, ldc=n + 3)
+    # k + 16 roundings of at most 2^-24 of what has been added up
+    ref, off = a[:, :k].double() @ w[:, :k].double().T, (a[:, :k].abs().double() @ w[:, :k].abs().double().T) * (k + 16) * 2.0 ** -24
+    if epi == _dense.EPI_GELU_GLU:
+        gate, up = ref[:, :n], ref[:, n:]
+        # |gelu'| < 1.2; tanh and the two products round by 2^-20 of a value of at most |gate|
+        off = 1.2 * off[:, :n] * up.abs() + (gate.abs() + 1.2 * off[:, :n]) * off[:, n:] + 2.0 ** -20 * (gate * up).abs()
+        ref = gelu_tanh(gate) * up
+    assert bool(((got - ref).abs() <= off + 1e-30).all())
