@@ -19,6 +19,7 @@
 #include "twm_dense_softmax_tc.cuh"
 #include "twm_dense_tc.cuh"
 #include "twm_dense_tc2.cuh"
+#include "twm_dense_tcs.cuh"
 
 namespace {
 
@@ -316,7 +317,7 @@ twm_status gemm_tc2_launch(const bf16* a, int lda, const bf16* w, int ldw, void*
 
 // Tile: the one whose waves cost least.  Measured time of one 64-K stage of a wave: 0.42, 0.25 and 0.20 us for tiles of
 // 128 rows x 256, 128 and 64 columns; 0.33 us for 256 x 256 on a pair of SMs (returned as 512).
-int tc_tile_choice(int M, int N, bool gated, int sms)
+int tc_tile_choice(int M, int N, bool gated, int sms, long* stage_cost)
 {
     int best = 256;
     long best_cost = -1;
@@ -330,7 +331,102 @@ int tc_tile_choice(int M, int N, bool gated, int sms)
     consider(256, 128, 256, sms, 42);
     consider(128, 128, 128, sms, 25);
     consider(64, 128, 64, sms, 20);
+    *stage_cost = best_cost;
     return best;
+}
+
+// ------------------------------------------------- product of few tiles --
+struct TcsPlan { int bn, splits, stages; };
+template <int BN>
+int tcs_stages(int bm, size_t limit) { return (int)std::min<size_t>(TS_MAX_STAGES, (limit - ts_smem_bytes<BN>(bm, 0, 1)) / ts_stage_bytes<BN>(bm)); }
+
+// Clusters of `splits` CTAs that run at once, one CTA to an SM.
+twm_status cluster_capacity(int splits, int* out)
+{
+    static int known[64][TS_MAX_SPLITS + 1] = {};
+    static std::mutex mutex;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return fail("cudaGetDevice", e);
+    std::lock_guard<std::mutex> lock(mutex);
+    int& n = known[dev][splits];
+    if (n == 0) {
+        auto kernel = gemm_tcs_kernel<128, TWM_EPI_STORE>;
+        const int smem = 200 * 1024;
+        if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return fail("gemm_tcs", e);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(splits);
+        cfg.blockDim = dim3(TC_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = splits;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if ((e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg)) != cudaSuccess) return fail("cudaOccupancyMaxActiveClusters", e);
+        n = std::max(n, 1);
+    }
+    *out = n;
+    return TWM_OK;
+}
+
+template <int BN, int EPI>
+twm_status gemm_tcs_launch(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, int M, int N, int K, const TcsPlan& plan, int flags,
+                           void* stream)
+{
+    constexpr bool gated = EPI == TWM_EPI_GELU_GLU;
+    constexpr int out = gated ? BN / 2 : BN;
+    TcsArgs g;
+    g.c = c; g.ldc = ldc; g.M = M; g.N = N; g.K = K;
+    g.m_tiles = (M + TC_BM - 1) / TC_BM;
+    g.bm = ((M + g.m_tiles - 1) / g.m_tiles + 7) / 8 * 8;
+    g.splits = plan.splits; g.stages = plan.stages;
+    if (!rows_map(&g.a_map, a, M, K, lda, g.bm) || !rows_map(&g.w_map, w, gated ? 2L * N : N, K, ldw, out))
+        return invalid("cuTensorMapEncodeTiled refused a map of the shared tcgen05 product");
+    return launch("gemm_tcs", gemm_tcs_kernel<BN, EPI>, dim3((unsigned)((long)g.m_tiles * ((N + out - 1) / out) * g.splits)), TC_THREADS,
+                  ts_smem_bytes<BN>(g.bm, g.stages, g.splits), flags, stream, g.splits > 1 ? g.splits : 0, g);
+}
+template <int EPI>
+twm_status gemm_tcs(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, int M, int N, int K, const TcsPlan& plan, int flags, void* stream)
+{
+    switch (plan.bn) {
+        case 256: return gemm_tcs_launch<256, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
+        case 128: return gemm_tcs_launch<128, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
+        default: return gemm_tcs_launch<64, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
+    }
+}
+
+// Whether the product of few tiles takes a call (bn > 0), and how; tile and stage_cost are tc_tile_choice's.
+// K shared by s CTAs: costs the stages of one share, 1/937 us for each of their rows but no less than 0.12 us, and 3.0 + 0.4 s us for
+// the exchange of the sums (fitted to 40 products of 4 to 700 rows: the choice is within 4 % of the best on average).  Clusters that
+// would not all run at once cost twice that, so they are not taken: 18 clusters of 8 do not fit 148 SMs.
+// Not shared, one CTA a tile: where the plain product would take one wave of 64- or 128-column tiles, which the even rows and
+// the single accumulator do no slower (2 rows, 8208 x 2048: 16.0 -> 9.1 us; 100 rows: 9.4 -> 9.0); and for up to 128 rows in several
+// waves, two CTAs to an SM so that one loads while the other stores (2 rows, 18944 gated x 3584: 50.7 -> 43.1 us; 100 rows: 47.6 ->
+// 46.4).  From 65 rows on and more than two CTAs an SM the persistent product is faster (128 rows, 152064 x 3584: 210 against 225 us).
+twm_status tcs_plan(int M, int N, int K, bool gated, int sms, int tile, long stage_cost, TcsPlan* plan)
+{
+    const int m_tiles = (M + TC_BM - 1) / TC_BM, bm = ((M + m_tiles - 1) / m_tiles + 7) / 8 * 8, k_tiles = (K + TC_BK - 1) / TC_BK;
+    auto tiles = [&](int bn) { return (long)m_tiles * ((N + (gated ? bn / 2 : bn) - 1) / (gated ? bn / 2 : bn)); };
+    const size_t one = 215 * 1024, two = 105 * 1024;                // shared memory of one and of two CTAs to an SM
+    auto stages = [&](int bn, size_t limit) { return bn == 64 ? tcs_stages<64>(bm, limit) : tcs_stages<128>(bm, limit); };
+    *plan = {0, 1, 0};
+    long best = stage_cost * k_tiles;
+    for (int bn = 64; bn <= 128; bn *= 2)
+        for (int s = 2; s <= std::min(TS_MAX_SPLITS, k_tiles); ++s) {
+            if (tiles(bn) * s > sms) break;
+            const long cost = (k_tiles + s - 1) / s * std::max(12L, (bm + bn) * 16L / 150) + 300 + 40 * s;
+            if (cost >= best) continue;
+            int fit = 0;
+            TRY(cluster_capacity(s, &fit));
+            if (tiles(bn) > fit) continue;
+            best = cost;
+            *plan = {bn, s, stages(bn, one)};
+        }
+    if (plan->bn == 0 && tile <= 128 && tiles(tile) <= sms) *plan = {tile, 1, stages(tile, one)};
+    if (plan->bn == 0 && m_tiles == 1 && (bm <= 64 || tiles(128) <= 2 * sms)) *plan = {128, 1, stages(128, two)};
+    return TWM_OK;
 }
 
 template <int EPI>
@@ -339,7 +435,13 @@ twm_status gemm_tc(const bf16* a, int lda, const bf16* w, int ldw, void* c, int 
 {
     int sms = 148;
     TRY(device(&sms));
-    if (width == 0) width = tc_tile_choice(M, N, EPI == TWM_EPI_GELU_GLU, sms);
+    if (width == 0) {
+        long stage_cost;
+        TcsPlan plan;
+        width = tc_tile_choice(M, N, EPI == TWM_EPI_GELU_GLU, sms, &stage_cost);
+        TRY(tcs_plan(M, N, K, EPI == TWM_EPI_GELU_GLU, sms, width, stage_cost, &plan));
+        if (plan.bn > 0) return gemm_tcs<EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
+    }
     switch (width) {
         case 512: return gemm_tc2_launch<EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
         case 256: return gemm_tc_launch<256, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);

@@ -77,3 +77,28 @@ def test_gemm_f32_edges(m, n, k, lda, ldw, epi):
         off = 1.2 * off[:, :n] * up.abs() + (gate.abs() + 1.2 * off[:, :n]) * off[:, n:] + 2.0 ** -20 * (gate * up).abs()
         ref = gelu_tanh(gate) * up
     assert bool(((got - ref).abs() <= off + 1e-30).all())
+
+
+@pytest.mark.parametrize("m,n,k,lda", [(1, 1, 1, 8), (1, 300, 8192, 8192), (7, 130, 200, 208), (8, 5120, 2048, 2048), (9, 2048, 1032, 1040),
+                                       (37, 64, 2048, 2048), (64, 700, 136, 136), (65, 33000, 72, 72), (97, 130, 6000, 6000), (100, 2048, 2048, 2048),
+                                       (128, 9500, 64, 64), (129, 520, 4104, 4104), (200, 2050, 640, 640), (333, 1001, 3000, 3000)])
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
+def test_gemm_few_tiles(m, n, k, lda, epi):
+    """Products of few tiles: K shared by clusters of two to eight CTAs or not shared, two CTAs to an SM, rows and columns past the tiles."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rows = 2 * n if epi == _dense.EPI_GELU_GLU else n
+    a = torch.full((m, lda), 1e30, device="cuda").bfloat16()
+    w = torch.full((rows, lda), 1e30, device="cuda").bfloat16()
+    a[:, :k] = torch.randn((m, k), generator=gen, device="cuda")
+    w[:, :k] = torch.randn((rows, k), generator=gen, device="cuda") / math.sqrt(k)
+    got = gemm(a[:, :k], w[:, :k], epi, 0, n, ldc=n + 3)
+    # exact products; k + 16 roundings (the tensor core may cut instead) of at most 2^-23 of what has been added up
+    ref, off = a[:, :k].double() @ w[:, :k].double().T, (a[:, :k].double().abs() @ w[:, :k].double().abs().T) * (k + 16) * 2.0 ** -23
+    if epi == _dense.EPI_GELU_GLU:
+        gate, up = ref[:, :n], ref[:, n:]
+        # |gelu'| < 1.2; tanh and the two products round by 2^-20 of a value of at most |gate|
+        off = 1.2 * off[:, :n] * up.abs() + (gate.abs() + 1.2 * off[:, :n]) * off[:, n:] + 2.0 ** -20 * (gate * up).abs()
+        ref = gelu_tanh(gate) * up
+    if epi != _dense.EPI_STORE_F32:
+        off = off + 2.0 ** -8 * ref.abs()
+    assert bool(((got - ref).abs() <= off + 1e-30).all())
