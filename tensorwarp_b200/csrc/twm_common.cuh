@@ -157,6 +157,22 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_addr, uint32_t ra
 __device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
 }
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
+}
+// Sum over the CTAs 0 ... n - 1 (up to eight) of a cluster, in that order, of the four floats at the same place of their shared
+// memory: every load is issued before the first sum.
+__device__ __forceinline__ float4 cluster_sum4(const float* local, int n) {
+    const uint32_t at = smem_u32(local);
+    float4 t[8], v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) if (i < n) t[i] = ld_cluster_f32x4(mapa_shared(at, i));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) if (i < n) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
+    return v;
+}
 // hardware barrier over every thread of every CTA of the cluster (like __syncthreads, not a spin)
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -4,8 +4,8 @@
 // Bound by reading W; before that by what one SM can take in (64 bytes a clock, activations included) where fewer tiles than SMs
 // leave the machine idle: the down product of a 2048-wide layer has 32 tiles of 64 columns.  The rows are spread evenly over the
 // row tiles (333 rows: three tiles of 112), and a stage holds no more of them: fewer bytes a stage, more stages.  Each CTA
-// of a cluster accumulates its share of K in TMEM and pushes the sums to the CTAs that own the rows (shared memory of the
-// cluster, where the stages were), which add them in rank order: the same result every time, no workspace.
+// of a cluster accumulates its share of K in TMEM and leaves the sums in its shared memory, where the stages were; each adds up its
+// share of the rows over the cluster in rank order: the same result every time, no workspace.
 //
 // Weights cold, against twm_dense_tc.cuh: 2048 x 8192, 100 rows: 26.3 -> 11.3 us (K over four), 333 rows: 27.6 -> 18.9; 3584 x 18944,
 // 100 rows: 59.8 -> 29.2 us (4.6 TB/s); 2048 x 2048, 100 rows: 8.6 -> 6.6; 5120 x 2048, 2 rows: 16.7 -> 6.7.  Tiles of 256 columns
@@ -32,7 +32,7 @@ struct TcsArgs {
 template <int BN>
 __host__ __device__ constexpr int ts_stage_bytes(int bm) { return (bm + BN) * TC_BK * 2; }
 template <int BN>
-__host__ __device__ constexpr int ts_sum_bytes() { return (TC_BM + TS_MAX_SPLITS) * (BN + 4) * 4; }
+__host__ __device__ constexpr int ts_sum_bytes() { return TC_BM * (BN + 4) * 4; }
 // the stages, what the last stage's MMA reads past its rows, and where the sums of the cluster come together
 template <int BN>
 size_t ts_smem_bytes(int bm, int stages, int splits)
@@ -180,38 +180,30 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
             }
         }
     } else {
-        // every CTA of the cluster has used its stages: the sums go to the CTAs that own the rows, which add them in rank order
+        // this CTA's MMAs have run: its sums go where its stages were, and each CTA adds up its share of the rows in rank order
         const int own = (rows + g.splits - 1) / g.splits;
-        float* sums = reinterpret_cast<float*>(ring);               // [splits][own][LD]
-        cluster_sync_all();
+        float* sums = reinterpret_cast<float*>(ring);               // [row][LD]
         if (reader) {
-            const int r = warp * 32 + lane, owner = min(r, rows - 1) / own;
-            const uint32_t to = mapa_shared(smem_u32(sums + ((size_t)rank * own + min(r, rows - 1) - owner * own) * LD), owner);
+            float* to = sums + (warp * 32 + lane) * LD;
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 uint32_t d[16];
                 tc::tmem_ld<16>(at + c0, d);
                 tc::tmem_wait_ld();
-                if (r < rows) {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4)
-                        st_cluster_f32x4(to + (c0 + j) * 4, make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3])));
-                }
+                for (int j = 0; j < 16; j += 4)
+                    *reinterpret_cast<float4*>(to + c0 + j) = make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
             }
         }
         cluster_sync_all();
         for (int i = tid; i < own * (OUT / 4); i += TC_THREADS) {
             const int r = i / (OUT / 4), col = (i - r * (OUT / 4)) * 4, m = rank * own + r;
             if (m >= rows || n0 + col >= g.N) continue;
-            const float* p = sums + (size_t)r * LD + col;
-            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int s = 0; s < g.splits; ++s, p += (size_t)own * LD) {
-                const float4 x = *reinterpret_cast<const float4*>(p);
-                v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-                if (GATED) {
-                    const float4 z = *reinterpret_cast<const float4*>(p + OUT);
-                    u[0] += z.x; u[1] += z.y; u[2] += z.z; u[3] += z.w;
-                }
+            const float4 x = cluster_sum4(sums + m * LD + col, g.splits);
+            float v[4] = {x.x, x.y, x.z, x.w}, u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (GATED) {
+                const float4 z = cluster_sum4(sums + m * LD + OUT + col, g.splits);
+                u[0] = z.x; u[1] = z.y; u[2] = z.z; u[3] = z.w;
             }
             if (GATED) {
 #pragma unroll
@@ -219,6 +211,7 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
             }
             tc_store4<EPI>(g.c, (size_t)(row0 + m) * g.ldc, n0 + col, g.N, v);
         }
+        cluster_sync_all();                                         // nobody leaves while its sums may still be read
     }
     tc::tc_fence_before();
     __syncthreads();

@@ -1,5 +1,5 @@
 // twm_gemm_tcr.cuh — the tcgen05 / TMEM W4A16 kernel for many activation rows and wide matrices
-// (65 ... 128 rows per launch, scale group 128, N of at least a wave of 256-column tiles).
+// (65 ... 256 rows per launch, scale group 128).
 //
 // twm_gemm_tcw.cuh keeps the weights exact: the MMA multiplies (q - 8) * 2^-24 and the FP32 scale
 // meets the accumulator once per 128-group, which costs a read-back of the accumulator per group,
@@ -19,7 +19,8 @@
 // FP16 multiply by the column's scale rounds once), then, after the last stage, read-back and store
 // (thread = activation row, 64 columns).  Warp 16: TMA producer.  Warp 17: MMA issuer.  K order inside an
 // 8-wide core is k0,k4,k1,k5,k2,k6,k3,k7 as in the other tcgen05 kernels (the pre-pass writes the
-// activations that way).  One CTA per SM (about 180 KB of shared memory), 256 TMEM columns.
+// activations that way).  Fewer tiles than SMs: K is cut into slices, a cluster of up to eight CTAs a tile (see twm_gemm_tcw.cuh); 200
+// rows, weights cold: N=4608, K=3584 53.4 us in one slice, 24.7 in six; N=3584: 53.6 and 23.2; N=18944: 54.6 and 36.9 in two.  One CTA per SM (about 180 KB of shared memory), 256 TMEM columns.
 #pragma once
 
 #include "twm_common.cuh"
@@ -71,6 +72,9 @@ struct Smem {
     int abort_flag;
 };
 
+static_assert(offsetof(Smem<1>, sc) >= tcw::SLICE_BYTES<NT> && offsetof(Smem<2>, sc) >= tcw::SLICE_BYTES<NT>,
+              "the sums of a cluster lie where the stages were");
+
 template <int RB>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ GemmParams p)
@@ -84,7 +88,8 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     const int warp = tid >> 5;
     const int lane = tid & 31;
     const int n0 = blockIdx.x * NT;
-    const int n_stages = p.nkb / SB;                         // the whole K: this kernel does not split it
+    // a K slice (of a cluster) is whole scale groups: an even number of stages
+    const int st0 = blockIdx.y * p.blocks_per_split / SB, n_stages = min(p.nkb - (int)blockIdx.y * p.blocks_per_split, p.blocks_per_split) / SB;
 
     if (tid == 0) {
         for (int s = 0; s < PSTAGES; ++s) { mbar_init(&sm.p_full[s], 1); mbar_init(&sm.p_empty[s], UNPACK_WARPS); }
@@ -106,10 +111,10 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         const int slot = st % PSTAGES;
         const bool with_scales = scale_bulk && (st & 1) == 0;
         mbar_arrive_expect_tx(&sm.p_full[slot], (uint32_t)(second_half ? P_STAGE_BYTES : P_HALF_BYTES) + (with_scales ? (uint32_t)NT * 2 : 0u));
-        tma_load_2d(&sm.packed[slot][0], &p.packed_map, n0 * 2, st * SB, &sm.p_full[slot]);
-        if (second_half) tma_load_2d(&sm.packed[slot][P_HALF_BYTES], &p.packed_map, (n0 + 128) * 2, st * SB, &sm.p_full[slot]);
+        tma_load_2d(&sm.packed[slot][0], &p.packed_map, n0 * 2, (st0 + st) * SB, &sm.p_full[slot]);
+        if (second_half) tma_load_2d(&sm.packed[slot][P_HALF_BYTES], &p.packed_map, (n0 + 128) * 2, (st0 + st) * SB, &sm.p_full[slot]);
         if (with_scales)
-            bulk_g2s(&sm.sc[(st >> 1) % SSTAGES][0], p.scales + (size_t)(st >> 1) * p.N + n0, (uint32_t)NT * 2, &sm.p_full[slot]);
+            bulk_g2s(&sm.sc[(st >> 1) % SSTAGES][0], p.scales + (size_t)((st0 + st) >> 1) * p.N + n0, (uint32_t)NT * 2, &sm.p_full[slot]);
     };
     if (warp == WARP_TMA) {
         // weights are constants: the first ring-full streams before the preceding kernel has finished
@@ -137,7 +142,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                         mbar_arrive_expect_tx(&sm.a_full[as], (uint32_t)C::A_STAGE_BYTES);
 #pragma unroll
                         for (int rb = 0; rb < RB; ++rb)         // rows 128 rb ...: 256 64-bit words further along a K core's row run
-                            tma_load_2d(&sm.a[as][rb * A_BLOCK_BYTES], &p.act_map, rb * MB * 2, ast * KCORES, &sm.a_full[as]);
+                            tma_load_2d(&sm.a[as][rb * A_BLOCK_BYTES], &p.act_map, rb * MB * 2, (st0 + ast) * KCORES, &sm.a_full[as]);
                         ++ast; progress = true;
                     }
                 }
@@ -198,7 +203,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
             if ((st & 1) == 0) {                               // a new 128-group: this column's scale, both halves of a register
                 uint16_t h = 0;
                 if (scale_bulk) h = sm.sc[(st >> 1) % SSTAGES][col];
-                else if (col_ok) h = __ldg(p.scales + (size_t)(st >> 1) * p.N + n0 + col);
+                else if (col_ok) h = __ldg(p.scales + (size_t)((st0 + st) >> 1) * p.N + n0 + col);
                 const uint32_t hh = (uint32_t)h | ((uint32_t)h << 16);
                 s2 = *reinterpret_cast<const __half2*>(&hh);
             }
@@ -245,6 +250,30 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         pdl_wait_prior_grids();                                // C may be read (or, with the accumulate flag, was written) by a kernel before
         ok = ok && (*abort_flag == 0);
         const int nb = n0 + cpart * RCOLS;
+        if (p.splits > 1) {
+            // The slices of a cluster add up, 128 rows at a time (a CTA whose waits ran out shows what it has, so that the
+            // cluster's barriers are met; the error word is set).
+            float* sums = reinterpret_cast<float*>(&sm.packed[0][0]);
+#pragma unroll 1
+            for (int rb = 0; rb < RB; ++rb) {
+                const int rows = min(MB, p.M - rb * MB);
+                const uint32_t lane_tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + rb * NT + cpart * RCOLS;
+                float* to = sums + (quarter * 32 + lane) * tcw::SLICE_LD<NT> + cpart * RCOLS;
+#pragma unroll 1
+                for (int c0 = 0; c0 < RCOLS; c0 += 16) {
+                    uint32_t d[16];
+                    tc::tmem_ld<16>(lane_tmem + c0, d);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(to + c0 + j) = make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
+                }
+                cluster_sync_all();
+                tcw::slice_sum_store<NT>(p, sums, rb * MB, rows, blockIdx.y, n0, tid, UNPACK_WARPS * 32);
+                cluster_sync_all();                            // the sums are overwritten, or the CTA leaves
+            }
+            ok = false;                                        // stored
+        }
 #pragma unroll 1
         for (int rb = 0; rb < RB && ok; ++rb) {
             const int m = rb * MB + quarter * 32 + lane;
@@ -302,6 +331,10 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                 }
             }
         }
+    }
+
+    if (p.splits > 1 && warp >= UNPACK_WARPS) {                // the other warps of the barriers above
+        for (int i = 0; i < 2 * RB; ++i) cluster_sync_all();
     }
 
     // ------------------------------------------------------------ teardown --

@@ -1,5 +1,5 @@
-// twm_gemm_tcw.cuh — the tcgen05 / TMEM W4A16 kernel for many activation rows (65 ... 128 per
-// launch, scale group 128).
+// twm_gemm_tcw.cuh — the tcgen05 / TMEM W4A16 kernel for many activation rows (65 ... 256 per
+// launch, grid z = block of 128 rows; scale group 128).
 //
 // twm_gemm_tc.cuh puts the CTA's 128 weight columns on the MMA's M dimension and the (few)
 // activation rows on N = 16 ... 64: right while the weight stream is the bound, but an MMA of
@@ -23,6 +23,11 @@
 // Warp roles: 0-7 read-back and store (TMEM lane quarter = warp & 3, column half = warp >> 2),
 // 8-11 unpack (thread = column), 12 TMA producer, 13 MMA issuer.  One CTA per SM (about 195 KB of
 // shared memory, all 512 TMEM columns: four accumulators).
+//
+// Where the tiles leave SMs idle, K is cut into slices of whole scale groups (grid y), a cluster of up to eight CTAs a tile, whose
+// sums add up over the cluster's shared memory.  Weights cold, 128 rows: N=3584, K=3584: 29.2 us in one slice, 14.4 in four;
+// K=18944: 122 and 38.9 us (64 in five slices through the workspace, whose partials and last arriver's sum cost 7 us a slice).
+// 200 rows, K=18944: 115 us as two such launches, 69 as one launch of 2 x 28 tiles in two slices.
 #pragma once
 
 #include "twm_common.cuh"
@@ -72,12 +77,55 @@ struct Smem {
     int is_last;
 };
 
+static_assert(ASTAGES * A_STAGE_BYTES >= MB * (NT + 4) * 4, "the sums of a cluster lie where the activation stages were");
+
 // D[128 x N] (+)= A[128 x 16] (shared memory) * B[N x 16]^T (shared memory)
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// ------------------------------------------------ K slices of a tile that are one cluster --
+// Each CTA leaves its sums [row][SLICE_LD] of COLS columns in its shared memory, where its stages were.  After a barrier of the
+// cluster each adds up its share of the rows in slice order, a warp along a row, and stores C.  (Pushing the sums from the threads
+// that hold them, a row each, moved 7 bytes a clock: 20 us for 256 rows x 256 columns.)
+constexpr int MAX_SLICES = 8;
+template <int COLS> constexpr int SLICE_LD = COLS + 4;
+template <int COLS> constexpr int SLICE_BYTES = MB * SLICE_LD<COLS> * 4;
+
+template <int COLS>
+__device__ __forceinline__ void slice_sum_store(const GemmParams& p, const float* sums, int row0, int rows, int rank, int n0, int tid, int threads) {
+    const int own = (rows + p.splits - 1) / p.splits;
+    for (int i = tid; i < own * (COLS / 4); i += threads) {
+        const int r = i / (COLS / 4), c = (i % (COLS / 4)) * 4, m = rank * own + r, n = n0 + c;
+        if (m >= rows || n >= p.N) continue;
+        const float4 t = cluster_sum4(sums + (size_t)m * SLICE_LD<COLS> + c, p.splits);
+        const float v[4] = {t.x, t.y, t.z, t.w};
+        const size_t off = (size_t)(row0 + m) * p.ldc + n;
+        const bool whole = n + 4 <= p.N && !p.accumulate;
+        if (p.c_is_f16) {
+            __half* cp = reinterpret_cast<__half*>(p.c) + off;
+            if (whole && (reinterpret_cast<uintptr_t>(cp) & 7) == 0) {
+                const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(cp) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < p.N) cp[j] = __float2half_rn(p.accumulate ? v[j] + __half2float(cp[j]) : v[j]);
+            }
+        } else {
+            float* cp = reinterpret_cast<float*>(p.c) + off;
+            if (whole && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+                *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < p.N) cp[j] = p.accumulate ? v[j] + cp[j] : v[j];
+            }
+        }
+    }
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -93,6 +141,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     const int b0 = blockIdx.y * p.blocks_per_split;          // a multiple of four (whole 128-groups, host plan)
     const int b1 = min(p.nkb, b0 + p.blocks_per_split);
     const int n_stages = (b1 - b0) / GROUP_BLOCKS;           // scale groups of this K slice
+    const int row0 = blockIdx.z * MB, rows = min(MB, p.M - row0);       // this CTA's rows
 
     if (tid == 0) {
         for (int s = 0; s < WSTAGES; ++s) { mbar_init(&sm.w_full[s], 1); mbar_init(&sm.w_empty[s], UNPACK_WARPS); }
@@ -143,7 +192,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                     const int as = ast % ASTAGES;
                     if (ast < ASTAGES || mbar_try_wait(&sm.a_empty[as], ((ast / ASTAGES) - 1) & 1)) {
                         mbar_arrive_expect_tx(&sm.a_full[as], (uint32_t)A_STAGE_BYTES);
-                        tma_load_2d(&sm.a[as][0], &p.act_map, 0, (b0 + ast * GROUP_BLOCKS) * 4, &sm.a_full[as]);
+                        tma_load_2d(&sm.a[as][0], &p.act_map, row0 * 2, (b0 + ast * GROUP_BLOCKS) * 4, &sm.a_full[as]);
                         ++ast; progress = true;
                     }
                 }
@@ -222,7 +271,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     } else {
         // ------------------------------------------------- read-back and store --
         const int quarter = warp & 3, half = warp >> 2;
-        const int m = quarter * 32 + lane;                   // this thread's activation row = its TMEM lane
+        const int m = row0 + quarter * 32 + lane;            // this thread's activation row; its TMEM lane
         const int cbase = half * EPI_COLS;                   // its first column inside the tile
         const uint32_t lane_tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + cbase;
         pdl_wait_prior_grids();                              // C may be read by the kernel before
@@ -272,7 +321,16 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         // this thread's 64 results are one contiguous run of its C row: 16-byte stores where the row allows
         const size_t row_off = (size_t)m * p.ldc + nb;
         const bool full = nb + EPI_COLS <= p.N;
-        if (ok && row_ok) {
+        if (p.cluster_reduce) {
+            // (a CTA whose waits ran out shows what it has, so that the cluster's barriers are met; the error word is set)
+            float* sums = reinterpret_cast<float*>(&sm.a[0][0]);       // this CTA's MMAs have run: its stages are free
+            float* to = sums + (m - row0) * SLICE_LD<NT> + cbase;
+#pragma unroll
+            for (int j = 0; j < EPI_COLS; j += 4) *reinterpret_cast<float4*>(to + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            cluster_sync_all();
+            slice_sum_store<NT>(p, sums, row0, rows, blockIdx.y, n0, tid, EPI_THREADS);
+            cluster_sync_all();                              // nobody leaves while its sums may still be read
+        } else if (ok && row_ok) {
             if (p.splits == 1) {
                 if (p.c_is_f16) {
                     __half* cp = reinterpret_cast<__half*>(p.c) + row_off;
@@ -327,7 +385,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                 }
             }
         }
-        if (p.splits > 1) {
+        if (p.splits > 1 && !p.cluster_reduce) {             // more slices than a cluster holds: through the workspace
             __threadfence();
             named_bar_sync(3, EPI_THREADS);
             if (tid == 0) {
@@ -376,6 +434,11 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                 if (tid == 0) atomicExch(&p.ws_counters[blockIdx.x], 0u);
             }
         }
+    }
+
+    if (p.cluster_reduce && warp >= WARP_UNPACK0) {          // the other warps of the two barriers above
+        cluster_sync_all();
+        cluster_sync_all();
     }
 
     // ------------------------------------------------------------ teardown --

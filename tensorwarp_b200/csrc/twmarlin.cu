@@ -282,10 +282,10 @@ int auto_kernel(int M, int N, int K, int G, bool a_is_f16, bool indirect, int sp
     // a wave of 256-column tiles, no K slices asked for) take the 256-column kernel, whose weights enter the tensor
     // core rounded to FP16 as in the reference's batched route; the others the exact-weight kernel, which can split K.
     if (M >= kTcwFromRows && G == 128 && N >= 128 && !indirect) {
-        // Measured on K=3584 (us, 128 / 256 rows): N=37888: tcr 43 / 60, tcw 56 / 111; N=28416: 44 / 60 against 56 / 112;
-        // N=18944: 44 / 59 against 32 / 60; N=9472: 42 / 56 against 30 / 60; N=4608: 41 / 55 against 29 / 59.  And K=18944,
-        // N=3584: tcr 182 (14 tiles, no K slices), tcw 64 in five slices.  So: more than one wave of 128-column
-        // tiles, or more than 128 rows, goes to the 256-column kernel unless K is long and the tiles are few.
+        // Measured on K=3584 (us, 128 / 256 rows, each with the K slices of its plan): N=37888: tcr 46 / 61, tcw 57 / 110; N=18944:
+        // 28 / 39 against 30 / 56; N=4608: 18 / 27 against 17 / 21.  K=18944, N=3584: 37 / 52 against 39 / 70.  So: more than one wave
+        // of 128-column tiles, or more than 128 rows, goes to the 256-column kernel unless K is long and the tiles are few, where
+        // the exact weights stay.
         const int tiles_w = (N + twm::tcw::NT - 1) / twm::tcw::NT, tiles_r = (N + twm::tcr::NT - 1) / twm::tcr::NT;
         const bool long_k_few_tiles = K >= 8192 && 4 * tiles_r <= kDefaultSms;
         const bool wide = (tiles_w > kDefaultSms || M > twm::tcw::MB) && !long_k_few_tiles && splits_override <= 1;
@@ -307,7 +307,7 @@ int resolve_kernel(const twm_gemm_args* a)
 }
 
 constexpr int kTcRows = 64;      // activation rows one tcgen05 launch carries
-constexpr int kTcwRows = twm::tcw::MB;   // ... and one wide tcgen05 launch
+constexpr int kTcwRows = 2 * twm::tcw::MB;   // ... and one wide tcgen05 launch (128 where K slices go through the workspace)
 constexpr int kTcrRows = 2 * twm::tcr::MB;   // ... and one 256-column tcgen05 launch (two blocks of 128 rows)
 
 twm_status launch_tcw(const twm::GemmParams& p, dim3 grid, bool pdl, cudaStream_t stream)
@@ -318,11 +318,19 @@ twm_status launch_tcw(const twm::GemmParams& p, dim3 grid, bool pdl, cudaStream_
     cfg.blockDim = dim3(twm::tcw::THREADS, 1, 1);
     cfg.dynamicSmemBytes = sizeof(twm::tcw::Smem);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.cluster_reduce) {                              // the K slices of a tile
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+        attr[n++].val.clusterDim.y = grid.y;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, twm::tcw::gemm_kernel, p);
     if (e != cudaSuccess) { set_error("launch tcw::gemm_kernel", e); return TWM_ELAUNCH; }
     return TWM_OK;
@@ -336,11 +344,19 @@ twm_status launch_tcr(const twm::GemmParams& p, int rows, dim3 grid, bool pdl, c
     cfg.blockDim = dim3(twm::tcr::THREADS, 1, 1);
     cfg.dynamicSmemBytes = rows > twm::tcr::MB ? sizeof(twm::tcr::Smem<2>) : sizeof(twm::tcr::Smem<1>);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.cluster_reduce) {                              // the K slices of a tile
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+        attr[n++].val.clusterDim.y = grid.y;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     cudaError_t e = rows > twm::tcr::MB ? cudaLaunchKernelEx(&cfg, twm::tcr::gemm_kernel<2>, p)
                                         : cudaLaunchKernelEx(&cfg, twm::tcr::gemm_kernel<1>, p);
     if (e != cudaSuccess) { set_error("launch tcr::gemm_kernel", e); return TWM_ELAUNCH; }
@@ -567,10 +583,32 @@ twm_status launch_mma_rows(twm::GemmParams& p, char* stage_buf, dim3 grid, unsig
     return go(twm::mma::gemm_rows_kernel<32, 2>, twm::mma::gemm_rows_kernel<32, 0>, sizeof(twm::mma::RowsSmem<32>));
 }
 
-// twm_plan; prepass (streaming MMA kernel's staging pre-pass) 0: not used (up to eight rows), 1: by the size rule,
+// Clusters of s CTAs, one CTA to an SM, that run at once.
+int resident_clusters(int s, int sm_count)
+{
+    static const int b200[twm::tcw::MAX_SLICES + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};      // cudaOccupancyMaxActiveClusters, 200 KB of shared memory
+    return sm_count == kDefaultSms ? b200[s] : 8 * (sm_count / 8 / s);
+}
+// Blocks per K slice of the tcgen05 kernels for many rows, whose slices are one cluster: as many slices as cost least, counted in
+// waves of a slice's scale groups (128 K each) and the exchange of the sums, which grows with the slices.
+int cluster_blocks(int tiles, int nkb, int sm_count, double group_us, double exchange_us)
+{
+    const int groups = nkb / 4;
+    int best_blocks = nkb;
+    double best = (double)((tiles + sm_count - 1) / sm_count) * groups * group_us;
+    for (int s = 2; s <= std::min(twm::tcw::MAX_SLICES, groups); ++s) {
+        const int per = (groups + s - 1) / s, fit = resident_clusters((groups + per - 1) / per, sm_count);
+        if (fit < 1) continue;
+        const double cost = (double)((tiles + fit - 1) / fit) * (per * group_us + exchange_us) + 0.3 * s;
+        if (cost < best) { best = cost; best_blocks = per * 4; }
+    }
+    return best_blocks;
+}
+
+// twm_plan; tcw_rows: rows a launch of the wide tcgen05 kernel carries; prepass (streaming MMA kernel's staging pre-pass) 0: not used (up to eight rows), 1: by the size rule,
 // 2: from two rows on whatever the size
 twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int splits_override,
-                     int kernel_override, int prepass, twm_plan_t* out)
+                     int kernel_override, int prepass, twm_plan_t* out, int tcw_rows = kTcwRows)
 {
     if (!out || !shape_ok(M, N, K, group_size)) return TWM_EINVAL;
     if (splits_override < 0 || splits_override > kMaxSplits) return TWM_EINVAL;
@@ -582,21 +620,28 @@ twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int spli
         kernel != TWM_KERNEL_TCR)
         return TWM_EINVAL;
     if ((kernel == TWM_KERNEL_TCW || kernel == TWM_KERNEL_TCR) && (group_size != 128 || N < 128)) return TWM_EINVAL;
-    if (kernel == TWM_KERNEL_TCR) {          // 256-column tiles over the whole K: no slices, no scratch but the reordered activations
+    if (kernel == TWM_KERNEL_TCR) {          // 256-column tiles; K slices only as a cluster: no scratch but the reordered activations
         if (splits_override > 1) return TWM_EINVAL;
-        const int rows_r = std::min(M, kTcrRows);
+        const int rows_r = std::min(M, kTcrRows), tiles = (N + twm::tcr::NT - 1) / twm::tcr::NT;
+        // a 128-K group costs 1.5 us (1.95 with two row blocks), an exchange of the slices' sums about 5 (7): fitted to 2048 ... 18944 K
+        const bool two = rows_r > twm::tcr::MB;
+        const int bps = splits_override == 1 ? nkb : cluster_blocks(tiles, nkb, sm_count, two ? 1.95 : 1.5, two ? 7.0 : 5.0);
         out->kernel = kernel;
         out->n_tile = twm::tcr::NT;
-        out->splits = 1;
-        out->blocks_per_split = K / 32;
-        out->grid_x = (N + twm::tcr::NT - 1) / twm::tcr::NT;
-        out->grid_y = 1;
+        out->splits = (nkb + bps - 1) / bps;
+        out->blocks_per_split = bps;
+        out->grid_x = tiles;
+        out->grid_y = out->splits;
         out->workspace_bytes = kCounterBytes + 256 + (size_t)rows_r * K * 2;
-        out->cluster_reduce = 0;
+        out->cluster_reduce = out->splits > 1 ? 1 : 0;
         return TWM_OK;
     }
+    // slices of whole scale groups that were asked for
+    auto asked_blocks = [&](int align) { return ((nkb + splits_override - 1) / splits_override + align - 1) / align * align; };
+    const bool tcw_workspace = kernel == TWM_KERNEL_TCW && splits_override > 0 &&
+                               (nkb + asked_blocks(4) - 1) / asked_blocks(4) > twm::tcw::MAX_SLICES;
     // rows one launch carries; more rows are served by further launches
-    const int rows = std::min(M, kernel == TWM_KERNEL_TC ? kTcRows : (kernel == TWM_KERNEL_TCW ? kTcwRows : (kernel == TWM_KERNEL_MMA ? mma_rows_for(M) : 8)));
+    const int rows = std::min(M, kernel == TWM_KERNEL_TC ? kTcRows : (kernel == TWM_KERNEL_TCW ? (tcw_workspace ? twm::tcw::MB : tcw_rows) : (kernel == TWM_KERNEL_MMA ? mma_rows_for(M) : 8)));
     const int n_tiles = (N + twm::simt::NT - 1) / twm::simt::NT;
     const int slots = kernel == TWM_KERNEL_TCW ? sm_count
                                                : sm_count * ((kernel != TWM_KERNEL_SIMT || mmax_for(rows) <= 4) ? 2 : 1);
@@ -606,25 +651,18 @@ twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int spli
     const bool can_cluster = (kernel == TWM_KERNEL_MMA) && rows <= twm::mma::CLUSTER_ROWS;
     int splits, bps;
     if (splits_override > 0) {
-        bps = (nkb + splits_override - 1) / splits_override;
-        bps = (bps + align - 1) / align * align;
+        bps = asked_blocks(align);
         if (bps > max_bps) return TWM_EINVAL;
         splits = (nkb + bps - 1) / bps;
     } else if (kernel == TWM_KERNEL_TCW) {
-        // Measured (128 rows): a 128-K stage costs about 0.8 us, a K slice about 7 us of its own (partials out, count,
-        // the last arriver's sum).  Slices pay only with few tiles and a long K: N=3584, K=18944: 124 us unsplit,
-        // 64 us in five slices; N=3584, K=3584: 29 us unsplit, 36 us in two.
-        const int stages = nkb / align;
-        int want = 1;
-        if (stages >= 64 && 2 * n_tiles <= slots) want = std::min(std::min(slots / n_tiles, stages / 28), kMaxSplits);
-        bps = (stages + want - 1) / want * align;
+        bps = cluster_blocks(n_tiles * ((rows + twm::tcw::MB - 1) / twm::tcw::MB), nkb, sm_count, 0.8, 4.0);
         splits = (nkb + bps - 1) / bps;
     } else {
         choose_splits(n_tiles, nkb, slots, sm_count, max_bps, align, can_cluster ? twm::mma::MAX_CLUSTER / rows : kMaxSplits,
                       can_cluster, &splits, &bps);
         if (bps > max_bps) return TWM_EINVAL;
     }
-    const bool cluster = can_cluster && splits > 1 && splits * rows <= twm::mma::MAX_CLUSTER;
+    const bool cluster = splits > 1 && (kernel == TWM_KERNEL_TCW ? splits <= twm::tcw::MAX_SLICES : can_cluster && splits * rows <= twm::mma::MAX_CLUSTER);
     out->kernel = kernel;
     out->n_tile = twm::simt::NT;
     out->splits = splits;
@@ -633,7 +671,7 @@ twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int spli
     out->grid_y = splits;
     out->workspace_bytes = (splits > 1 && !cluster) ? kCounterBytes + (size_t)splits * rows * N * sizeof(float) : 0;
     if (kernel == TWM_KERNEL_TC || kernel == TWM_KERNEL_TCW)    // + the launch's activations in the MMA's K order, behind the split-K part
-        out->workspace_bytes = kCounterBytes + (splits > 1 ? (size_t)splits * rows * N * sizeof(float) : 0) + 256 + (size_t)rows * K * 2;
+        out->workspace_bytes = kCounterBytes + (splits > 1 && !cluster ? (size_t)splits * rows * N * sizeof(float) : 0) + 256 + (size_t)rows * K * 2;
     if (kernel == TWM_KERNEL_MMA && (mma_prepass(rows, K, N) || (prepass == 2 && rows >= 2))) {      // + the rows staged as B fragments with their group sums
         if (prepass)
             out->workspace_bytes = kCounterBytes + (splits > 1 ? (size_t)splits * rows * N * sizeof(float) : 0) + 256 + mma_rows_stage_bytes(rows, K, group_size);
@@ -708,8 +746,15 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
         prepass = 0;                             // the CTAs' own stager warps
     }
     twm_plan_t pl;
+    int tcw_rows = kTcwRows;
     st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, prepass, &pl);
     if (st != TWM_OK) return st;
+    if (kernel == TWM_KERNEL_TCW && a->workspace_bytes < pl.workspace_bytes) {       // room for fewer rows at a time
+        tcw_rows = twm::tcw::MB;
+        st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, prepass, &pl, tcw_rows);
+        if (st != TWM_OK) return st;
+    }
+    if (kernel == TWM_KERNEL_TCW && pl.splits > 1 && !pl.cluster_reduce) tcw_rows = twm::tcw::MB;
     if (prepass == 1 && a->M <= 8 && (!a->workspace || a->workspace_bytes < pl.workspace_bytes)) {
         prepass = 0;                             // no room for the staged rows: the stager warps need none
         st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, 0, &pl);
@@ -720,7 +765,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
         // The reference's call has no scratch argument (its split-K adds into C with atomics,
         // quantize.rs:1337-1357).  A caller that passes none still gets its GEMM: one K slice per
         // tile, nothing to add up, at the price of fewer CTAs on small N.
-        st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, 1, kernel, prepass, &pl);
+        st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, 1, kernel, prepass, &pl, tcw_rows);
         if (st != TWM_OK) return st;
     }
     if (pl.workspace_bytes > 0) {
@@ -742,7 +787,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
     const size_t a_elt = a->a_dtype == TWM_F16 ? 2 : 4;
     const size_t c_elt = a->c_dtype == TWM_F16 ? 2 : 4;
     if ((kernel == TWM_KERNEL_TCW || kernel == TWM_KERNEL_TCR) && (a->packed_offsets != nullptr || a->comm)) return TWM_EINVAL;
-    const int row_step = kernel == TWM_KERNEL_TC ? kTcRows : (kernel == TWM_KERNEL_TCW ? kTcwRows : (kernel == TWM_KERNEL_TCR ? kTcrRows : (kernel == TWM_KERNEL_MMA ? mma_rows_for(a->M) : 8)));
+    const int row_step = kernel == TWM_KERNEL_TC ? kTcRows : (kernel == TWM_KERNEL_TCW ? tcw_rows : (kernel == TWM_KERNEL_TCR ? kTcrRows : (kernel == TWM_KERNEL_MMA ? mma_rows_for(a->M) : 8)));
     CUtensorMap packed_map;
     int map_rows = 0;
     if (a->packed_offsets == nullptr && a->N >= 128 && kernel != TWM_KERNEL_SIMT) {
@@ -762,7 +807,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
         p.ws_partials = a->workspace ? (float*)((char*)a->workspace + kCounterBytes) : nullptr;
         p.splits = pl.splits; p.blocks_per_split = pl.blocks_per_split;
         p.reduce_slices = pl.splits;
-        p.cluster_reduce = (pl.cluster_reduce && rows <= twm::mma::CLUSTER_ROWS) ? 1 : 0;
+        p.cluster_reduce = (pl.cluster_reduce && (kernel != TWM_KERNEL_MMA || rows <= twm::mma::CLUSTER_ROWS)) ? 1 : 0;
         p.accumulate = (a->flags & TWM_FLAG_ACCUMULATE) ? 1 : 0;
         p.no_wait = ((a->flags & TWM_FLAG_INDEPENDENT) && (a->flags & TWM_FLAG_PDL) && kernel == TWM_KERNEL_MMA &&
                      pl.workspace_bytes == 0 && !p.accumulate && a->packed_offsets == nullptr && !a->comm) ? 1 : 0;
@@ -789,14 +834,14 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
             }
             st = launch_prepass((__half*)xp, (const __half*)p.a, p.lda, rows, a->K, a->flags, stream_);
             if (st != TWM_OK) return st;
-            st = launch_tcr(p, rows, dim3(pl.grid_x, 1, 1), pdl, stream);
+            st = launch_tcr(p, rows, dim3(pl.grid_x, pl.grid_y, 1), pdl, stream);
         }
         else if (kernel == TWM_KERNEL_TCW) {
             if (!map_rows) {
                 snprintf(t_last_error, sizeof(t_last_error), "cuTensorMapEncodeTiled failed for the packed map of the wide tcgen05 kernel");
                 return TWM_ELAUNCH;
             }
-            const size_t part_bytes = pl.splits > 1 ? (size_t)pl.splits * std::min(a->M, kTcwRows) * a->N * sizeof(float) : 0;
+            const size_t part_bytes = pl.splits > 1 && !p.cluster_reduce ? (size_t)pl.splits * std::min(a->M, tcw_rows) * a->N * sizeof(float) : 0;
             char* xp = (char*)a->workspace + kCounterBytes + ((part_bytes + 255) / 256) * 256;
             if (!make_act_map_wide(&p.act_map, xp, rows, a->K)) {
                 snprintf(t_last_error, sizeof(t_last_error), "cuTensorMapEncodeTiled failed for the activation map");
@@ -804,7 +849,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
             }
             st = launch_prepass((__half*)xp, (const __half*)p.a, p.lda, rows, a->K, a->flags, stream_);
             if (st != TWM_OK) return st;
-            st = launch_tcw(p, dim3(pl.grid_x, pl.grid_y, 1), pdl, stream);
+            st = launch_tcw(p, dim3(pl.grid_x, pl.grid_y, (rows + twm::tcw::MB - 1) / twm::tcw::MB), pdl, stream);
         }
         else if (kernel == TWM_KERNEL_TC) {
             // pre-pass: this launch's rows in [K/8][rows][8] order, then the GEMM loads them by TMA
@@ -866,6 +911,10 @@ twm_status twm_gemm_w4a16_static_ws(const twm_gemm_args* a, void* stream_)
     twm_plan_t pl;
     st = twm_plan(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, &pl);
     if (st != TWM_OK) return st;
+    if (pl.workspace_bytes > kStaticWsBytes && kernel == TWM_KERNEL_TCW) {
+        st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, 1, &pl, twm::tcw::MB);
+        if (st != TWM_OK) return st;
+    }
     if (pl.workspace_bytes > kStaticWsBytes && kernel == TWM_KERNEL_MMA && a->M <= 8) {
         // as twm_gemm_w4a16 will: up to eight rows can do without the staging pre-pass
         st = plan_impl(a->M, a->N, a->K, a->group_size, sm_count, a->splits_override, kernel, 0, &pl);

@@ -348,6 +348,31 @@ def test_256_column_tensor_core_kernel(m, k, n):
         _run_gemm(a, packed, scales, m, n, k, group, torch.float16, torch.float32, kernel_override=kern, splits_override=2)
 
 
+@pytest.mark.parametrize("kernel,m,k,n,splits", [(_lib.TWM_KERNEL_TCW, 256, 1024, 300, 8), (_lib.TWM_KERNEL_TCW, 200, 1152, 130, 9), (_lib.TWM_KERNEL_TCW, 200, 1280, 130, 9), (_lib.TWM_KERNEL_TCW, 129, 384, 1000, 3),
+                                                 (_lib.TWM_KERNEL_TCR, 256, 1152, 258, 0), (_lib.TWM_KERNEL_TCR, 70, 1664, 1001, 0), (_lib.TWM_KERNEL_TCR, 129, 2048, 4700, 0)])
+@pytest.mark.parametrize("c_dtype", [torch.float16, torch.float32])
+def test_many_rows_in_slices(kernel, m, k, n, splits, c_dtype):
+    """K slices of a cluster and (from nine on) through the workspace: the accumulate flag, rows of C off 16 bytes, and a
+    workspace that has room for 128 rows only."""
+    group = 128
+    _, packed, scales = _quantised(k, n, group, 61)
+    a = seeded_activations(m, k, 5)
+    ref = oracle.w4a16_f64(a, packed, scales, m, n, k, group, weights_f16=kernel == _lib.TWM_KERNEL_TCR)
+    assert kernel == _lib.TWM_KERNEL_TCW or q.plan(m, n, k, group, kernel_override=kernel).splits > 1
+    need = [q.plan(r, n, k, group, kernel_override=kernel, splits_override=splits).workspace_bytes for r in (128, m)]
+    p, s = _to_dev(packed, torch.uint8), _to_dev(scales.view(np.int16), torch.int16)
+    outs = []
+    for size in (need if kernel == _lib.TWM_KERNEL_TCW else need[1:]):
+        c = torch.full((m, n + 3), 2.0, dtype=c_dtype, device=DEV)
+        q.gemm_tw_marlin(_to_dev(a, torch.float16), p, s, c[:, :n], m, n, k, group_size=group, workspace=q.Workspace(size), kernel_override=kernel,
+                         splits_override=splits, flags=_lib.TWM_FLAG_ACCUMULATE)
+        torch.cuda.synchronize()
+        assert q.device_error() == 0 and bool((c[:, n:] == 2.0).all())
+        outs.append(c[:, :n].float().cpu().numpy() - 2.0)
+    for y in outs:
+        assert _abs_err_over_rms(y, ref) < 4 * TC_ABS_F32 + (2.0 ** -10 * (np.abs(ref).max() + 2) / np.sqrt(np.mean(ref ** 2)) if c_dtype == torch.float16 else 0)
+
+
 def test_wide_tensor_core_kernel_refuses_what_it_cannot_do():
     k, n = 256, 256
     _, packed, scales = _quantised(k, n, 32, 46)
