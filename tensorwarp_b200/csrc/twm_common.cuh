@@ -162,15 +162,18 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr) {
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
     return v;
 }
-// Sum over the CTAs 0 ... n - 1 (up to eight) of a cluster, in that order, of the four floats at the same place of their shared
-// memory: every load is issued before the first sum.
+// Sum over the CTAs 0 ... n - 1 of a cluster, in that order, of the four floats at the same place of their shared memory: eight
+// loads are issued before the first sum.
 __device__ __forceinline__ float4 cluster_sum4(const float* local, int n) {
     const uint32_t at = smem_u32(local);
-    float4 t[8], v = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = 0; b < n; b += 8) {
+        float4 t[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) if (i < n) t[i] = ld_cluster_f32x4(mapa_shared(at, i));
+        for (int i = 0; i < 8; ++i) if (b + i < n) t[i] = ld_cluster_f32x4(mapa_shared(at, b + i));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) if (i < n) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
+        for (int i = 0; i < 8; ++i) if (b + i < n) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
+    }
     return v;
 }
 // hardware barrier over every thread of every CTA of the cluster (like __syncthreads, not a spin)
@@ -286,6 +289,33 @@ struct GemmParams {
     const uint8_t* rows_b;
     const float* rows_asum;
 };
+
+// Four consecutive results of C's row m from column n on (accumulate: added to what C holds).
+__device__ __forceinline__ void store_c4(const GemmParams& p, int m, int n, const float4 r) {
+    const float v[4] = {r.x, r.y, r.z, r.w};
+    const size_t off = (size_t)m * p.ldc + n;
+    const bool whole = n + 4 <= p.N && !p.accumulate;
+    if (p.c_is_f16) {
+        __half* cp = reinterpret_cast<__half*>(p.c) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(cp) & 7) == 0) {
+            const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+            *reinterpret_cast<uint2*>(cp) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < p.N) cp[j] = __float2half_rn(p.accumulate ? v[j] + __half2float(cp[j]) : v[j]);
+        }
+    } else {
+        float* cp = reinterpret_cast<float*>(p.c) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+            *reinterpret_cast<float4*>(cp) = r;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < p.N) cp[j] = p.accumulate ? v[j] + cp[j] : v[j];
+        }
+    }
+}
 
 // ---- row-parallel output pushed to the tensor-parallel peers (GemmParams::n_peers != 0) ----
 // One value of the FP32 result, element `off` of the [M, ldc] output: a plain store into every

@@ -101,30 +101,7 @@ __device__ __forceinline__ void slice_sum_store(const GemmParams& p, const float
     for (int i = tid; i < own * (COLS / 4); i += threads) {
         const int r = i / (COLS / 4), c = (i % (COLS / 4)) * 4, m = rank * own + r, n = n0 + c;
         if (m >= rows || n >= p.N) continue;
-        const float4 t = cluster_sum4(sums + (size_t)m * SLICE_LD<COLS> + c, p.splits);
-        const float v[4] = {t.x, t.y, t.z, t.w};
-        const size_t off = (size_t)(row0 + m) * p.ldc + n;
-        const bool whole = n + 4 <= p.N && !p.accumulate;
-        if (p.c_is_f16) {
-            __half* cp = reinterpret_cast<__half*>(p.c) + off;
-            if (whole && (reinterpret_cast<uintptr_t>(cp) & 7) == 0) {
-                const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
-                *reinterpret_cast<uint2*>(cp) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (n + j < p.N) cp[j] = __float2half_rn(p.accumulate ? v[j] + __half2float(cp[j]) : v[j]);
-            }
-        } else {
-            float* cp = reinterpret_cast<float*>(p.c) + off;
-            if (whole && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
-                *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (n + j < p.N) cp[j] = p.accumulate ? v[j] + cp[j] : v[j];
-            }
-        }
+        store_c4(p, row0 + m, n, cluster_sum4(sums + (size_t)m * SLICE_LD<COLS> + c, p.splits));
     }
 }
 

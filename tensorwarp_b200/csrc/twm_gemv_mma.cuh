@@ -596,7 +596,8 @@ gemv_kernel(const __grid_constant__ GemmParams p)
 // row itself would cost more than the multiply (16 rows of K = 3584 are 114 KB per CTA), so a pre-pass
 // (stage_rows_kernel) writes the B fragments and the group sums once, in the stagers' layout, to the
 // workspace, and one lane per CTA copies a ring stage's share of them with bulk copies, next to the
-// producer warp's weights.  Arithmetic and summation order are those of gemv_kernel.
+// producer warp's weights.  Arithmetic and summation order are those of gemv_kernel.  Up to eight K slices are a
+// cluster whose CTAs add up over its shared memory; more, and those pushed to tensor-parallel peers, go through the workspace.
 
 constexpr int rows_stages(int mp) { return mp <= 8 ? 5 : (mp <= 16 ? 4 : 3); }    // ring depth that leaves two CTAs per SM
 
@@ -828,7 +829,11 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
 
     // ----------------------------------------------------- store / split-K --
     // lane (g, t): C[m = 8 nt + 2t, + 1][n = n0 + wcol + g] and the same rows for column + 8
-    if (warp >= CONSUMER_WARPS) return;
+    if (warp >= CONSUMER_WARPS) {
+        __syncwarp();
+        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers below
+        return;
+    }
     const int nA = n0 + wcol + g, nB = nA + 8;
     // tensor-parallel push: this launch's sequence number and buffer set (only the consumer kernel advances it)
     const unsigned int comm_seq = p.n_peers ? ld_volatile_u32(p.comm_state) : 0u;
@@ -847,6 +852,25 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
         }
     };
     named_bar_sync(1, CONSUMERS);
+    if (p.cluster_reduce) {
+        // the slices of the tile are one cluster: each CTA adds up a share of the rows over it, in slice order
+        constexpr int LD = NT + 4;
+        static_assert(sizeof(sm.packed) >= MP * LD * sizeof(float), "the sums lie where the weights were");
+        float* sums = reinterpret_cast<float*>(&sm.packed[0][0]);
+#pragma unroll
+        for (int nt = 0; nt < NTL; ++nt) {
+            float* to = sums + (nt * 8 + 2 * t) * LD + wcol + g;
+            to[0] = tot[nt][0]; to[LD] = tot[nt][1]; to[8] = tot[nt][2]; to[LD + 8] = tot[nt][3];
+        }
+        cluster_sync_all();
+        if (*abort_flag == 0)
+            for (int i = blockIdx.y * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
+                const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+                if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));
+            }
+        cluster_sync_all();                                  // nobody leaves while its sums may still be read
+        return;
+    }
     // a wait expired: leave C untouched, the error word is set; with peers the CTA still counts itself, so that
     // their consumers do not wait for this rank in vain
     if (*abort_flag && !p.n_peers) return;

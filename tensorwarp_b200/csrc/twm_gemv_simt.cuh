@@ -25,7 +25,8 @@
 // reduction.  Nibbles 6 and 7 of a word reach into the exponent field, so
 // they are taken from `v >> 8`.
 //
-// Split-K.  Slices write FP32 partials to the caller's workspace; the CTA that
+// Split-K.  Up to sixteen slices of up to four rows are a cluster, whose CTAs each add up a share of the columns in slice order from one
+// another's shared memory (one row, 3072 x 2048: 7.4 -> 5.4 us).  Others write FP32 partials to the caller's workspace; the CTA that
 // arrives last on the tile's counter adds the slices in slice order (so the
 // result does not depend on arrival order), stores C and puts the counter back
 // to zero.  No memset launch, no atomics on C.
@@ -146,6 +147,7 @@ gemv_kernel(const GemmParams p)
             }
             __syncwarp();
         }
+        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers at the end
         return;
     }
 
@@ -269,7 +271,7 @@ gemv_kernel(const GemmParams p)
 
     // ------------------------------------------- reduce the eight warps --
     named_bar_sync(1, CONSUMERS);
-    if (*abort_flag) return;   // a wait expired: leave C untouched, the error word is set
+    if (*abort_flag && !p.cluster_reduce) return;   // a wait expired: leave C untouched, the error word is set
     float* red = reinterpret_cast<float*>(&sm.packed[0][0]);   // [SB][MMAX][NT], ring is idle now
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -279,7 +281,7 @@ gemv_kernel(const GemmParams p)
 
     const int n = n0 + tid;
     const bool owner = (tid < NT) && (n < p.N);
-    float part[MMAX];
+    float part[MMAX] = {};
     if (owner) {
 #pragma unroll
         for (int m = 0; m < MMAX; ++m) {
@@ -309,6 +311,23 @@ gemv_kernel(const GemmParams p)
             for (int m = 0; m < MMAX; ++m)
                 if (m < p.M) store_c(m, part[m]);
         }
+        return;
+    }
+
+    if (p.cluster_reduce) {
+        // the slices of the tile are one cluster: each CTA adds up a share of the columns over it, in slice order
+        float* sums = red + SB * MMAX * NT;                  // [row][NT], this slice's
+        if (tid < NT) {
+#pragma unroll
+            for (int m = 0; m < MMAX; ++m) sums[m * NT + tid] = part[m];
+        }
+        cluster_sync_all();
+        if (*abort_flag == 0)
+            for (int i = tid * p.splits + blockIdx.y; i < p.M * (NT / 4); i += CONSUMERS * p.splits) {
+                const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+                if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * NT + c, p.splits));
+            }
+        cluster_sync_all();                                  // nobody leaves while its sums may still be read
         return;
     }
 

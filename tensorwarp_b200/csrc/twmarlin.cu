@@ -38,6 +38,8 @@ void set_error(const char* where, cudaError_t e)
 constexpr int kMaxDevices = 64;
 constexpr int kDefaultSms = 148;
 constexpr int kMaxSplits = 64;
+// K slices that add up as a cluster, at most: staged rows of the streaming kernel, and up to four rows of the FP32 kernel
+constexpr int kMaxStagedSlices = 8, kMaxSimtSlices = 16;
 constexpr size_t kCounterBytes = 16384;   // 4096 tile counters at the head of the workspace
 
 // Dynamic shared memory of a tcgen05 launch.  Each CTA allocates 256 of the SM's 512 tensor-memory
@@ -85,6 +87,12 @@ twm_status ensure_device(int* sm_count_out)
             raise((const void*)twm::simt::gemv_kernel<2>);
             raise((const void*)twm::simt::gemv_kernel<4>);
             raise((const void*)twm::simt::gemv_kernel<8>);
+            auto wide_cluster = [&](const void* fn) {
+                if (r == cudaSuccess) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            };
+            wide_cluster((const void*)twm::simt::gemv_kernel<1>);
+            wide_cluster((const void*)twm::simt::gemv_kernel<2>);
+            wide_cluster((const void*)twm::simt::gemv_kernel<4>);
             auto raise_tc = [&](const void* fn, size_t bytes) {
                 if (r == cudaSuccess)
                     r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -220,9 +228,11 @@ bool shape_ok(int M, int N, int K, int G)
 // `cluster` = the slices of a tile will be launched as one thread-block cluster.  A cluster
 // lives inside one GPC (8 GPCs share the SMs), so a slice count that does not pack into a
 // GPC's CTA slots costs a second wave: that is counted here.
+// `two_resident` = ... and two of its CTAs share an SM: as many clusters at once as cudaOccupancyMaxActiveClusters said.
 void choose_splits(int n_tiles, int nkb, int slots, int sm_count, int max_bps, int align, int max_splits, bool cluster,
-                   int* splits, int* bps)
+                   bool two_resident, int* splits, int* bps)
 {
+    static const int b200[17] = {0, 296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14};      // by cluster size, 100 KB a CTA
     double best = 1e30;
     int best_s = 1, best_bps = nkb;
     const int smax = std::min(max_splits, nkb);
@@ -239,7 +249,7 @@ void choose_splits(int n_tiles, int nkb, int slots, int sm_count, int max_bps, i
             // slot "layer" at a time, so a GPC of 18 SMs with two slots per SM holds
             // 2 * floor(18 / s) clusters (4 of size 7, not 5).
             const int sms_per_gpc = sm_count / 8;
-            const long resident_clusters = 8L * (slots / sm_count) * (sms_per_gpc / s_eff);
+            const long resident_clusters = two_resident && sm_count == kDefaultSms ? b200[s_eff] : 8L * (slots / sm_count) * (sms_per_gpc / s_eff);
             if (resident_clusters == 0) continue;
             waves = std::max(waves, ((long)n_tiles + resident_clusters - 1) / resident_clusters);
         }
@@ -442,11 +452,19 @@ twm_status launch_simt(const twm::GemmParams& p, int mmax, dim3 grid, bool pdl, 
     cfg.blockDim = dim3(twm::simt::THREADS, 1, 1);
     cfg.dynamicSmemBytes = sizeof(twm::simt::Smem);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.cluster_reduce) {                              // the K slices of a tile
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+        attr[n++].val.clusterDim.y = grid.y;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     cudaError_t e;
     switch (mmax) {
         case 1: e = cudaLaunchKernelEx(&cfg, twm::simt::gemv_kernel<1>, p); break;
@@ -495,21 +513,36 @@ twm_status static_ws_address(void** out)
 namespace {
 constexpr int kArgmaxParts = 592;   // 4 CTAs per SM
 
+// cluster_y > 0: the CTAs of grid y form a cluster
 template <typename... KArgs, typename... Args>
-twm_status launch_op(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int flags,
-                     void* stream_, Args... args)
+twm_status launch_cluster(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int flags, unsigned cluster_y,
+                          void* stream_, Args... args)
 {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)stream_;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (flags & TWM_FLAG_PDL) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster_y > 0) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+        attr[n++].val.clusterDim.y = cluster_y;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = (flags & TWM_FLAG_PDL) ? 1 : 0;
+    cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (e != cudaSuccess) { set_error(name, e); return TWM_ELAUNCH; }
     return TWM_OK;
+}
+template <typename... KArgs, typename... Args>
+twm_status launch_op(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int flags,
+                     void* stream, Args... args)
+{
+    return launch_cluster(name, kernel, grid, block, smem, flags, 0, stream, args...);
 }
 
 // twm_gemm_args.next: which bytes the GEMM after this one starts with, under its own plan.
@@ -574,8 +607,9 @@ twm_status launch_mma_rows(twm::GemmParams& p, char* stage_buf, dim3 grid, unsig
         st = p.a_kind == 0 ? stage(twm::mma::stage_rows_kernel<0, 0>) : (p.a_kind == 1 ? stage(twm::mma::stage_rows_kernel<0, 1>) : stage(twm::mma::stage_rows_kernel<0, 2>));
     if (st != TWM_OK) return st;
     auto go = [&](auto k128, auto k32, size_t smem) {
-        return p.group == 128 ? launch_op("mma::gemm_rows_kernel", k128, grid, dim3(twm::mma::THREADS), smem, flags & TWM_FLAG_PDL, stream, p)
-                              : launch_op("mma::gemm_rows_kernel", k32, grid, dim3(twm::mma::THREADS), smem, flags & TWM_FLAG_PDL, stream, p);
+        const unsigned cluster = p.cluster_reduce ? grid.y : 0;
+        return p.group == 128 ? launch_cluster("mma::gemm_rows_kernel", k128, grid, dim3(twm::mma::THREADS), smem, flags & TWM_FLAG_PDL, cluster, stream, p)
+                              : launch_cluster("mma::gemm_rows_kernel", k32, grid, dim3(twm::mma::THREADS), smem, flags & TWM_FLAG_PDL, cluster, stream, p);
     };
     if (mp == 8) return go(twm::mma::gemm_rows_kernel<8, 2>, twm::mma::gemm_rows_kernel<8, 0>, sizeof(twm::mma::RowsSmem<8>));
     if (mp == 16) return go(twm::mma::gemm_rows_kernel<16, 2>, twm::mma::gemm_rows_kernel<16, 0>, sizeof(twm::mma::RowsSmem<16>));
@@ -658,8 +692,11 @@ twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int spli
         bps = cluster_blocks(n_tiles * ((rows + twm::tcw::MB - 1) / twm::tcw::MB), nkb, sm_count, 0.8, 4.0);
         splits = (nkb + bps - 1) / bps;
     } else {
-        choose_splits(n_tiles, nkb, slots, sm_count, max_bps, align, can_cluster ? twm::mma::MAX_CLUSTER / rows : kMaxSplits,
-                      can_cluster, &splits, &bps);
+        // The slices of staged rows and of up to four rows of the FP32 kernel are a cluster too, though room in the workspace is asked
+        // for.  (Five to eight FP32 rows, one CTA to an SM: six slices of a cluster 44 us, eighteen through the workspace 31.)
+        const bool staged = kernel == TWM_KERNEL_MMA && prepass == 1 && mma_prepass(rows, K, N), simt = kernel == TWM_KERNEL_SIMT && mmax_for(rows) <= 4;
+        const int most = can_cluster ? twm::mma::MAX_CLUSTER / rows : staged ? kMaxStagedSlices : simt ? kMaxSimtSlices : kMaxSplits;
+        choose_splits(n_tiles, nkb, slots, sm_count, max_bps, align, most, can_cluster || staged || simt, staged || simt, &splits, &bps);
         if (bps > max_bps) return TWM_EINVAL;
     }
     const bool cluster = splits > 1 && (kernel == TWM_KERNEL_TCW ? splits <= twm::tcw::MAX_SLICES : can_cluster && splits * rows <= twm::mma::MAX_CLUSTER);
@@ -702,8 +739,9 @@ size_t twm_workspace_bytes(int M, int N, int K, int group_size)
     if (twm_plan(M, N, K, group_size, kDefaultSms, 0, TWM_KERNEL_SIMT, &simt) == TWM_OK)
         need = std::max(need, simt.workspace_bytes);
     // (the streaming MMA kernel with its staging pre-pass whatever the size: a push to peers asks for it)
-    if (plan_impl(M, N, K, group_size, kDefaultSms, 0, TWM_KERNEL_MMA, 2, &simt) == TWM_OK)
-        need = std::max(need, simt.workspace_bytes);
+    for (int prepass = 1; prepass <= 2; ++prepass)
+        if (plan_impl(M, N, K, group_size, kDefaultSms, 0, TWM_KERNEL_MMA, prepass, &simt) == TWM_OK)
+            need = std::max(need, simt.workspace_bytes);
     return need;
 }
 
@@ -808,6 +846,9 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
         p.splits = pl.splits; p.blocks_per_split = pl.blocks_per_split;
         p.reduce_slices = pl.splits;
         p.cluster_reduce = (pl.cluster_reduce && (kernel != TWM_KERNEL_MMA || rows <= twm::mma::CLUSTER_ROWS)) ? 1 : 0;
+        const bool staged = kernel == TWM_KERNEL_MMA && prepass && rows >= (prepass == 2 ? 2 : 3);
+        if (staged) p.cluster_reduce = pl.splits > 1 && pl.splits <= kMaxStagedSlices && !a->comm;
+        if (kernel == TWM_KERNEL_SIMT) p.cluster_reduce = pl.splits > 1 && pl.splits <= kMaxSimtSlices && mmax_for(a->M) <= 4;
         p.accumulate = (a->flags & TWM_FLAG_ACCUMULATE) ? 1 : 0;
         p.no_wait = ((a->flags & TWM_FLAG_INDEPENDENT) && (a->flags & TWM_FLAG_PDL) && kernel == TWM_KERNEL_MMA &&
                      pl.workspace_bytes == 0 && !p.accumulate && a->packed_offsets == nullptr && !a->comm) ? 1 : 0;
@@ -864,7 +905,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
             if (st != TWM_OK) return st;
             st = launch_tc(p, rows, dim3(pl.grid_x, pl.grid_y, 1), pdl, stream);
         }
-        else if (kernel == TWM_KERNEL_MMA && prepass && rows >= (prepass == 2 ? 2 : 3)) {
+        else if (staged) {
             const size_t part_bytes = pl.splits > 1 ? (size_t)pl.splits * std::min(a->M, row_step) * a->N * sizeof(float) : 0;
             char* stage = (char*)a->workspace + kCounterBytes + ((part_bytes + 255) / 256) * 256;
             st = launch_mma_rows(p, stage, dim3(pl.grid_x, pl.grid_y, 1), a->flags, stream);

@@ -720,3 +720,26 @@ def test_tensor_parallel_shard_shapes(k, n):
     if (k, n) == (8192, 1280):
         p = q.plan(1, n, k, group)
         assert p.splits == 16 and p.cluster_reduce == 1
+
+
+@pytest.mark.parametrize("m,k,n,group,splits,f32", [(1, 512, 130, 32, 16, True), (2, 608, 64, 32, 7, True), (4, 4096, 300, 128, 0, True), (3, 1024, 129, 128, 9, True),
+                                                    (5, 1024, 200, 32, 3, True), (1, 544, 40, 32, 17, True), (9, 1024, 300, 32, 8, False), (24, 1152, 129, 128, 9, False),
+                                                    (31, 2048, 258, 128, 0, False)])
+def test_few_rows_in_slices(m, k, n, group, splits, f32):
+    """K slices that are a cluster (FP32 rows up to four, staged rows up to eight slices) and those that are not: ragged
+    columns, the accumulate flag, rows of C off 16 bytes, and the same bits every time."""
+    kern, dt = (_lib.TWM_KERNEL_SIMT, torch.float32) if f32 else (_lib.TWM_KERNEL_MMA, torch.float16)
+    _, packed, scales = _quantised(k, n, group, 67)
+    a = seeded_activations(m, k, 8)
+    ref = oracle.w4a16_f64(a, packed, scales, m, n, k, group)
+    p, s, ad = _to_dev(packed, torch.uint8), _to_dev(scales.view(np.int16), torch.int16), _to_dev(a, dt)
+    ws = q.Workspace(q.plan(m, n, k, group, kernel_override=kern, splits_override=splits).workspace_bytes)
+    outs = []
+    for flags in (0, _lib.TWM_FLAG_PDL, _lib.TWM_FLAG_ACCUMULATE):
+        c = torch.full((m, n + 1), 1.0, dtype=torch.float32, device=DEV)
+        q.gemm_tw_marlin(ad, p, s, c[:, :n], m, n, k, group_size=group, workspace=ws, kernel_override=kern, splits_override=splits, flags=flags)
+        torch.cuda.synchronize()
+        assert q.device_error() == 0 and bool((c[:, n:] == 1.0).all())
+        outs.append(c[:, :n].cpu().numpy())
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0] + np.float32(1), outs[2])
+    assert _abs_err_over_rms(outs[0], ref) < TC_ABS_F32
