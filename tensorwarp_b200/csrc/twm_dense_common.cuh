@@ -74,6 +74,17 @@ __device__ __forceinline__ float group_sum(float v, float* red, int threads, int
     for (int w = 0; w < (threads >> 5); ++w) t += red[w];
     return t;
 }
+// two sums at once (`red` holds 64 floats), each as group_sum gives it
+__device__ __forceinline__ float2 group_sum2(float v, float w, float* red, int threads, int bar) {
+    v = ops::warp_sum(v);
+    w = ops::warp_sum(w);
+    named_bar_sync(bar, threads);
+    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = v; red[32 + (threadIdx.x >> 5)] = w; }
+    named_bar_sync(bar, threads);
+    float2 t = make_float2(0.0f, 0.0f);
+    for (int i = 0; i < (threads >> 5); ++i) { t.x += red[i]; t.y += red[32 + i]; }
+    return t;
+}
 __device__ __forceinline__ float inv_rms(float sumsq, int n, float eps) { return 1.0f / sqrtf(sumsq / (float)n + eps); }
 
 // True in one lane of a converged warp.  Code under it is known to run in one thread, which the tensor-core and TMA

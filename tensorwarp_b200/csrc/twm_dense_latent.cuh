@@ -239,11 +239,38 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
     const int per_cta = (g.vdim_pad + splits - 1) / splits;
     const T* w_uk = g.w_expand + (size_t)h * g.dim_pad * g.rank_pad + first;
     const T* w_uv = g.w_expand + (size_t)g.heads * g.dim_pad * g.rank_pad + (size_t)h * g.vdim_pad * g.rank_pad;
-    if (own > 0)
+    // the weights into registers where a thread's share is small: they are constants
+    constexpr int LK = 4, LR = 2, LC = 2;
+    const int vecs = own > 0 ? (own + V::N - 1) / V::N : 1;
+    const int vpp = min(vecs, LD_THREADS);                     // column vectors at a time
+    const int groups = max(1, LD_THREADS / vpp);
+    const bool early_k = own > 0 && vecs <= LD_THREADS && groups * LK >= g.dim_pad;
+    const bool early_v = per_cta <= LR * (LD_THREADS / 32) && g.rank_pad / V::N <= LC * 32;
+    const int v_first = rank * per_cta, v_end = min(g.vdim_pad, v_first + per_cta);
+    uint4 wk[LK], wv[LR][LC];
+#pragma unroll
+    for (int j = 0; j < LK; ++j) {
+        const int d = tid / vpp + j * groups;
+        wk[j] = early_k && tid / vpp < groups && d < g.dim_pad
+                    ? __ldg(reinterpret_cast<const uint4*>(w_uk + (tid % vpp) * V::N + (size_t)d * g.rank_pad)) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int r = 0; r < LR; ++r)
+#pragma unroll
+        for (int j = 0; j < LC; ++j) {
+            const int e = v_first + warp + r * (LD_THREADS / 32), c = lane + j * 32;
+            wv[r][j] = early_v && e < v_end && c < g.rank_pad / V::N ? __ldg(reinterpret_cast<const uint4*>(w_uv + (size_t)e * g.rank_pad) + c)
+                                                                   : make_uint4(0, 0, 0, 0);
+        }
+    if (own > 0 && !early_k)
         for (int i = tid; i < g.dim_pad; i += LD_THREADS)
             for (int c = 0; c < own * (int)sizeof(T); c += 128) l2_prefetch(reinterpret_cast<const uint8_t*>(w_uk + (size_t)i * g.rank_pad) + c);
-    for (int e = rank * per_cta + tid; e < min(g.vdim_pad, (rank + 1) * per_cta); e += LD_THREADS)
+    for (int e = v_first + tid; e < v_end && !early_v; e += LD_THREADS)
         l2_prefetch_bulk(w_uv + (size_t)e * g.rank_pad, (uint32_t)(g.rank_pad * sizeof(T)));
+    constexpr int LN = 2;                                          // a thread's first columns of the newest token's latent
+    float nw[LN];
+#pragma unroll
+    for (int j = 0; j < LN; ++j) nw[j] = tid + j * LD_THREADS < g.rank_pad ? __ldg(g.norm + tid + j * LD_THREADS) : 0.0f;
     if (h == 0) {
         const int now = min(max(*(volatile const int*)g.meta, 0), g.capacity - 1), from = max(0, now - g.window + 1), share_now = (now - from) / splits + 1;
         const T* rows_now = g.cache + (size_t)*(volatile const int*)(g.meta + 1) * g.capacity * width;
@@ -270,6 +297,11 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
 
     // ---- the query: rotated part, and this CTA's share of the mapped part ----
     const float* q = g.proj + h * qw;
+    const float* down = g.proj + g.heads * qw;
+    float dn[LN];                                                  // asked for before the first use, as is the gate
+#pragma unroll
+    for (int j = 0; j < LN; ++j) dn[j] = newest && tid + j * LD_THREADS < g.rank_pad ? down[tid + j * LD_THREADS] : 0.0f;
+    const float gate_in = g.proj[g.heads * qw + width + h];
     for (int d = tid; d < g.dim_pad; d += LD_THREADS) qu[d] = q[d];
     for (int i = tid; i < half; i += LD_THREADS) {
         const float2 o = rotate_pair(make_float2(q[g.dim_pad + 2 * i], q[g.dim_pad + 2 * i + 1]), g.rot_table[(size_t)p * half + i]);
@@ -279,13 +311,21 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
     __syncthreads();
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");    // every CTA of the cluster has started
     {
-        const int vecs = own > 0 ? (own + V::N - 1) / V::N : 1;
-        const int vpp = min(vecs, LD_THREADS);                     // column vectors at a time
-        const int groups = max(1, LD_THREADS / vpp);
         for (int v0 = 0; v0 * V::N < own; v0 += vpp) {
             const int vi = v0 + tid % vpp, dg = tid / vpp;
             float acc[V::N] = {};
-            if (dg < groups && vi < vecs) {
+            if (early_k) {
+#pragma unroll
+                for (int j = 0; j < LK; ++j) {
+                    const int d = dg + j * groups;
+                    if (dg >= groups || d >= g.dim_pad) continue;
+                    float f[V::N];
+                    V::unpack(wk[j], f);
+                    const float qd = qu[d];
+#pragma unroll
+                    for (int e = 0; e < V::N; ++e) acc[e] = fmaf(f[e], qd, acc[e]);
+                }
+            } else if (dg < groups && vi < vecs) {
                 const T* w = w_uk + vi * V::N;
 #pragma unroll 4
                 for (int d = dg; d < g.dim_pad; d += groups) {
@@ -313,10 +353,11 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
     }
     // ---- the newest token ----
     float kir = 1.0f;
-    const float* down = g.proj + g.heads * qw;
     if (newest) {
         float ss = 0.0f;
-        for (int i = tid; i < g.rank_pad; i += LD_THREADS) ss = fmaf(down[i], down[i], ss);
+#pragma unroll
+        for (int j = 0; j < LN; ++j) ss = fmaf(dn[j], dn[j], ss);
+        for (int i = tid + LN * LD_THREADS; i < g.rank_pad; i += LD_THREADS) ss = fmaf(down[i], down[i], ss);
         kir = inv_rms(group_sum(ss, red, LD_THREADS, 1), g.rank, g.eps);
     }
     for (int i = tid; i < share; i += LD_THREADS) os[i] = 0.0f;
@@ -332,11 +373,15 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
         if (newest && t0 + n == t_end) {
             T* mine = reinterpret_cast<T*>(rows + (size_t)(n - 1) * stride);
             T* kept = h == 0 && p < g.capacity ? cache + (size_t)p * width : nullptr;
-            for (int i = tid; i < g.rank_pad; i += LD_THREADS) {
-                const T v = from_f32<T>(down[i] * kir * __ldg(g.norm + i));
+            auto keep = [&](int i, float x, float w) {
+                const T v = from_f32<T>(x * kir * w);
                 mine[i] = v;
                 if (kept != nullptr) kept[i] = v;
-            }
+            };
+#pragma unroll
+            for (int j = 0; j < LN; ++j)
+                if (tid + j * LD_THREADS < g.rank_pad) keep(tid + j * LD_THREADS, dn[j], nw[j]);
+            for (int i = tid + LN * LD_THREADS; i < g.rank_pad; i += LD_THREADS) keep(i, down[i], __ldg(g.norm + i));
             for (int i = tid; i < half; i += LD_THREADS) {
                 const float* k = down + g.rank_pad + 2 * i;
                 const float2 o = rotate_pair(make_float2(k[0], k[1]), g.rot_table[(size_t)p * half + i]);
@@ -418,8 +463,28 @@ latent_decode_kernel(const LatentDecodeArgs<T> g)
         qa[i] = o / sum;
     }
     __syncthreads();
-    const float gate = sigmoid_f32(g.proj[g.heads * qw + width + h]);
-    for (int e = rank * per_cta + warp; e < min(g.vdim_pad, (rank + 1) * per_cta); e += LD_THREADS / 32) {
+    const float gate = sigmoid_f32(gate_in);
+    if (early_v) {
+#pragma unroll
+        for (int r = 0; r < LR; ++r) {
+            const int e = v_first + warp + r * (LD_THREADS / 32);
+            if (e >= v_end) break;                                 // the warp's
+            float s = 0.0f;
+#pragma unroll
+            for (int j = 0; j < LC; ++j) {
+                const int c = lane + j * 32;
+                if (c >= g.rank_pad / V::N) break;
+                float f[V::N];
+                V::unpack(wv[r][j], f);
+#pragma unroll
+                for (int k = 0; k < V::N; ++k) s = fmaf(f[k], qa[c * V::N + k], s);
+            }
+            s = ops::warp_sum(s);
+            if (lane == 0) g.out[h * g.vdim_pad + e] = s * gate;
+        }
+        return;
+    }
+    for (int e = v_first + warp; e < v_end; e += LD_THREADS / 32) {
         float s = 0.0f;
         for (int c = lane; c < g.rank_pad / V::N; c += 32) {
             float f[V::N];
