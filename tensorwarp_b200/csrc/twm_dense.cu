@@ -11,6 +11,7 @@
 #include "twm_dense_common.cuh"
 #include "twm_dense_decode.cuh"
 #include "twm_dense_f32.cuh"
+#include "twm_dense_f32tc.cuh"
 #include "twm_dense_gla.cuh"
 #include "twm_dense_latent.cuh"
 #include "twm_dense_moe.cuh"
@@ -464,37 +465,48 @@ twm_status gemm_tc_any(const bf16* a, int lda, const bf16* w, int ldw, void* c, 
     return invalid("epilogue");
 }
 
-// The FP32 product on 16-byte copies.  Rows are spread evenly over tiles of up to 64; K over as many CTAs of a cluster as
-// cost least, counted in stages of 32 K: waves of two CTAs to an SM, and eight stages' time for the exchange of the sums.
-template <int TM, int EPI>
-twm_status gemm_f32_launch(const GemmF32Args& g, int n_tiles, int flags, void* stream)
-{
-    return launch("gemm_f32", gemm_f32_kernel<TM, EPI>, dim3((unsigned)((long)n_tiles * g.m_tiles * g.splits)), F32_THREADS, f32_smem_bytes(TM),
-                  flags, stream, g.splits > 1 ? g.splits : 0, g);
-}
+// The FP32 product of up to eight rows on 16-byte copies.  K over as many CTAs of a cluster as cost least, counted in stages of
+// 32 K: waves of two CTAs to an SM, and eight stages' time for the exchange of the sums.
 template <int EPI>
 twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, int ldc, int M, int N, int K, int flags, void* stream)
 {
     int sms = 148;
     TRY(device(&sms));
-    GemmF32Args g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, (M + 63) / 64, 1};
+    GemmF32Args g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, 1, 1};
     const int out = EPI == TWM_EPI_GELU_GLU ? F32_BN / 2 : F32_BN, n_tiles = (N + out - 1) / out, k_tiles = (K + F32_BK - 1) / F32_BK;
-    const int tm = ((M + g.m_tiles - 1) / g.m_tiles + 7) / 8;
     long best = -1;
     for (int s = 1; s <= F32_MAX_SPLITS; ++s) {
-        const long waves = ((long)n_tiles * g.m_tiles * s + 2 * sms - 1) / (2 * sms), cost = waves * ((k_tiles + s - 1) / s + (s > 1 ? 8 : 0));
+        const long waves = ((long)n_tiles * s + 2 * sms - 1) / (2 * sms), cost = waves * ((k_tiles + s - 1) / s + (s > 1 ? 8 : 0));
         if (best < 0 || cost < best) { best = cost; g.splits = s; }
     }
-    switch (tm) {
-        case 1: return gemm_f32_launch<1, EPI>(g, n_tiles, flags, stream);
-        case 2: return gemm_f32_launch<2, EPI>(g, n_tiles, flags, stream);
-        case 3: return gemm_f32_launch<3, EPI>(g, n_tiles, flags, stream);
-        case 4: return gemm_f32_launch<4, EPI>(g, n_tiles, flags, stream);
-        case 5: return gemm_f32_launch<5, EPI>(g, n_tiles, flags, stream);
-        case 6: return gemm_f32_launch<6, EPI>(g, n_tiles, flags, stream);
-        case 7: return gemm_f32_launch<7, EPI>(g, n_tiles, flags, stream);
-        default: return gemm_f32_launch<8, EPI>(g, n_tiles, flags, stream);
+    return launch("gemm_f32", gemm_f32_kernel<1, EPI>, dim3((unsigned)((long)n_tiles * g.splits)), F32_THREADS, f32_smem_bytes(1), flags, stream,
+                  g.splits > 1 ? g.splits : 0, g);
+}
+// From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 5 rows 2.37 / 2.72,
+// 9 rows 2.80 / 2.75, 20 rows 3.33 / 2.84, 70 rows 6.45 / 3.51, 256 rows 18.2 / 8.1; error against 64 bits of 70 rows x 2048 x 8192:
+// 4.1e-7 / 1.5e-7.
+constexpr int F32TC_ROWS = 9;
+
+// K over as many CTAs of a cluster as cost least, counted in stages of 64 K (about 1 us): waves of the clusters that run at once, and
+// four stages' time for the exchange of the sums.
+template <int EPI>
+twm_status gemm_f32tc(const float* a, int lda, const float* w, int ldw, void* c, int ldc, int M, int N, int K, int flags, void* stream)
+{
+    int sms = 148;
+    TRY(device(&sms));
+    GemmFxArgs g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, (M + FX_MAX_ROWS - 1) / FX_MAX_ROWS, 0, 1};
+    g.bm = ((M + g.m_tiles - 1) / g.m_tiles + 15) / 16 * 16;
+    const int out = EPI == TWM_EPI_GELU_GLU ? FX_BN / 2 : FX_BN, k_tiles = (K + FX_BK - 1) / FX_BK;
+    const long tiles = (long)((N + out - 1) / out) * g.m_tiles;
+    double best = (double)((tiles + sms - 1) / sms) * k_tiles;
+    for (int s = 2; s <= std::min(TS_MAX_SPLITS, k_tiles); ++s) {
+        int fit = 1;
+        TRY(cluster_capacity(s, &fit));
+        const double cost = (double)((tiles + fit - 1) / fit) * ((k_tiles + s - 1) / s + 4) + 0.3 * s;
+        if (cost < best) { best = cost; g.splits = s; }
     }
+    return launch("gemm_f32tc", gemm_f32tc_kernel<EPI>, dim3((unsigned)(tiles * g.splits)), FX_THREADS, fx_smem_bytes(g.bm), flags, stream,
+                  g.splits, g);
 }
 // rows that start on 16-byte boundaries
 bool f32_fits(const float* a, int lda, const float* w, int ldw)
@@ -505,6 +517,9 @@ bool f32_fits(const bf16*, int, const bf16*, int) { return false; }
 twm_status gemm_f32_any(const bf16*, int, const bf16*, int, void*, int, int, int, int, int, int, void*) { return invalid("the FP32 product takes float"); }
 twm_status gemm_f32_any(const float* a, int lda, const float* w, int ldw, void* c, int ldc, int M, int N, int K, int epi, int flags, void* stream)
 {
+    if (M >= F32TC_ROWS)
+        return epi == TWM_EPI_GELU_GLU ? gemm_f32tc<TWM_EPI_GELU_GLU>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream)
+                                       : gemm_f32tc<TWM_EPI_STORE_F32>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream);
     return epi == TWM_EPI_GELU_GLU ? gemm_f32<TWM_EPI_GELU_GLU>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream)
                                    : gemm_f32<TWM_EPI_STORE_F32>(a, lda, w, ldw, c, ldc, M, N, K, flags, stream);
 }

@@ -1,18 +1,15 @@
-// twm_dense_f32.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models, in true FP32.
+// twm_dense_f32.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models for up to eight rows, in FP32 FMAs.
 //
-// Bound by FP32 FMAs (72 TFLOP/s) from some thirty rows on, by reading W below.  Tile 8 TM rows x 128 weight rows, 32 K a stage, three
+// Bound by reading W.  Tile 8 TM rows x 128 weight rows, 32 K a stage, three
 // stages of 16-byte asynchronous copies, two CTAs to an SM.  A thread has TM x 4 sums, each as a PAIR over even and odd K
 // (fma.rn.f32x2: two FMAs an instruction), so both operands stay in shared memory as they lie in global memory, rows of K
 // padded by 16 bytes: a quarter warp reads eight consecutive rows without conflicts, and an operand needs no transposition.
-// TM is chosen so that the rows fill their tiles (70 rows: two tiles of 40 and not two of 64).
 //
 // Products with few tiles share K out over a cluster of up to eight CTAs.  Each pushes its sums to the CTAs that own the rows
 // (shared memory of the cluster), which add them in rank order: same result every time, no workspace.
 //
-// 70 rows, down product 2048 x 8192, weights cold: 684 -> 89 us (2 rows: 705 -> 41; 1024 rows: 2138 -> 938, 37 TFLOP/s), and the
-// error against 64 bits 1.6e-6 -> 4e-7.  Before: the tiles of twm_dense_simt.cuh, which copy element by element with nothing in
-// flight, 64 CTAs at 70 rows; those stay for rows that are not on 16-byte boundaries.  256 weight rows a tile with 8 x 8
-// sums a thread: 227 instead of 240 us at 256 rows, 167 instead of 88 at 70.
+// 2 rows, down product 2048 x 8192, weights cold: 705 -> 41 us against the tiles of twm_dense_simt.cuh, which copy element by element
+// with nothing in flight; those stay for rows that are not on 16-byte boundaries.  More rows: twm_dense_f32tc.cuh.
 #pragma once
 
 #include "twm_dense_common.cuh"

@@ -1,0 +1,258 @@
+// twm_dense_f32tc.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models on the tensor cores, with the error of an FP32 product.
+//
+// Every FP32 number is exactly the sum of three bfloat16 numbers: its leading eight bits, the next eight, the last eight (cut, so
+// that all have its sign).  A product of two is the sum of nine; the six largest are taken, the others are below 2^-21 of it
+// (2^-24 on average).  The tensor core multiplies them exactly, but cuts when it adds.  So the products of the leading parts (acc 0)
+// and the other five (acc 1, 2^-7 smaller) have accumulators of their own, and both are taken out and added up in FP32
+// registers every 64 K.
+//
+// Tile: 128 weight rows (the MMA's M) x up to 128 activation rows, 64 K a stage, two stages, one CTA to an SM, K shared by a
+// cluster of up to eight.  Warps 0-7 take accumulators out (thread = weight row, every second chunk of 16 activation rows),
+// 8-15 read FP32 rows from global memory, split them and write the six operands to shared memory, 16 issues the MMAs.  A stage moves
+// 160 KB through shared memory at 80 rows (24 MMAs read 6.5 KB each), which is what bounds it.
+//
+// A number that is not finite has no such sum.  The splitting threads notice one (what a number leaves behind its leading
+// part is then not a number), and the cluster computes its tile with plain FP32 FMAs instead.
+#pragma once
+
+#include "twm_dense_f32.cuh"
+#include "twm_dense_tcs.cuh"
+
+namespace twm {
+namespace dense {
+
+constexpr int FX_BN = 128, FX_BK = 64, FX_MAX_ROWS = 128, FX_CORES = FX_BK / 8;
+constexpr int FX_READERS = 256, FX_SPLITTERS = 256, FX_THREADS = FX_READERS + FX_SPLITTERS + 32, FX_LD = FX_BN + 4;
+// an operand part: [K core of 8][row][16 bytes], cores 16 bytes apart so that eight threads on a row write to distinct banks
+__host__ __device__ constexpr int fx_core_bytes(int rows) { return rows * 16 + 16; }
+__host__ __device__ constexpr int fx_part_bytes(int rows) { return FX_CORES * fx_core_bytes(rows); }
+__host__ __device__ constexpr int fx_stage_bytes(int bm) { return 3 * (fx_part_bytes(FX_BN) + fx_part_bytes(bm)); }
+inline size_t fx_smem_bytes(int bm) { return std::max(2 * fx_stage_bytes(bm), bm * FX_LD * 4) + 128; }
+
+struct GemmFxArgs {
+    const float *a, *w;
+    float* c;
+    int lda, ldw, ldc, M, N, K;     // gated: N output columns, 2 N weight rows
+    int m_tiles, bm, splits;        // bm: activation rows a tile, a multiple of 16
+};
+
+template <int EPI>
+__global__ void __launch_bounds__(FX_THREADS, 1)
+gemm_f32tc_kernel(const GemmFxArgs g)
+{
+    constexpr bool GATED = EPI == TWM_EPI_GELU_GLU;
+    constexpr int OUT = GATED ? FX_BN / 2 : FX_BN;
+    extern __shared__ __align__(128) uint8_t fx_smem[];
+    __shared__ __align__(8) uint64_t full[2], empty[2], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_s;
+    __shared__ __align__(16) float odd_s[4];         // [0]: not zero where a number was not finite
+    volatile int* abort_flag = &abort_s;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x % g.splits, tile = blockIdx.x / g.splits;
+    const int m0 = tile % g.m_tiles * g.bm, n0 = tile / g.m_tiles * OUT, rows = min(g.bm, g.M - m0);
+    const int k_tiles = (g.K + FX_BK - 1) / FX_BK;
+    const int k_first = (int)((long)rank * k_tiles / g.splits), steps = (int)((long)(rank + 1) * k_tiles / g.splits) - k_first;
+    const int stage_bytes = fx_stage_bytes(g.bm), w_part = fx_part_bytes(FX_BN), a_part = fx_part_bytes(g.bm);
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&full[i], FX_SPLITTERS / 32); mbar_init(&empty[i], 1);
+            mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], FX_READERS / 32);
+        }
+        abort_s = 0;
+        odd_s[0] = odd_s[1] = odd_s[2] = odd_s[3] = 0.0f;
+        mbar_fence_init();
+    }
+    if (warp == FX_THREADS / 32 - 1) {
+        tc::tmem_alloc(&tmem_s, 512);
+        tc::tc_fence_before();
+    }
+    __syncthreads();
+    tc::tc_fence_after();
+    pdl_launch_dependents();
+    const uint32_t tmem = tmem_s;
+    float acc[64];                                    // readers: sums of chunks 2 i + (warp >> 2)
+
+    if (warp == FX_THREADS / 32 - 1) {
+        // ------------------------------------------------------------ MMAs --
+        if (elect_one()) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bm >> 3) << 17) | ((uint32_t)(FX_BN >> 4) << 24);
+            const uint32_t w_core = fx_core_bytes(FX_BN), a_core = fx_core_bytes(g.bm);
+            bool ok = true;
+            for (int t = 0; t < steps && ok; ++t) {
+                const int s = t & 1;
+                if (!mbar_wait_bounded(&full[s], (t >> 1) & 1, abort_flag)) { ok = false; break; }
+                if (t >= 2 && !mbar_wait_bounded(&acc_empty[s], ((t >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                tc::tc_fence_after();
+                const uint32_t base = smem_u32(fx_smem + s * stage_bytes);
+                // (part of W, part of A): the leading parts into accumulator 0, the five next smaller products into 1
+                auto product = [&](int wp, int ap, uint32_t d, bool first) {
+                    uint64_t wd = tc::make_b_desc(base + wp * w_part, w_core, 128), ad = tc::make_b_desc(base + 3 * w_part + ap * a_part, a_core, 128);
+                    const uint64_t w_step = (2 * w_core) >> 4, a_step = (2 * a_core) >> 4;
+#pragma unroll
+                    for (int h = 0; h < FX_BK / 16; ++h) {
+                        tcw::mma_ss(d, wd, ad, idesc, first && h == 0 ? 0u : 1u);
+                        wd += w_step;
+                        ad += a_step;
+                    }
+                };
+                const uint32_t d = tmem + s * 256;
+                product(0, 0, d, true);
+                product(0, 2, d + 128, true);
+                product(2, 0, d + 128, false);
+                product(1, 1, d + 128, false);
+                product(0, 1, d + 128, false);
+                product(1, 0, d + 128, false);
+                tc::tc_commit(&empty[s]);
+                tc::tc_commit(&acc_full[s]);
+            }
+        }
+        __syncwarp();
+    } else if (warp >= FX_READERS / 32) {
+        // ------------------------------------------------------- splitting --
+        const int st = tid - FX_READERS, row0 = st >> 3, core = st & 7;      // rows row0 + 32 j, eight K each
+        float4 x[8][2];                               // 0-3: weight rows, 4-7: activation rows
+        auto load = [&](int j, int t) {
+            const int r = row0 + (j & 3) * 32, k = (k_first + t) * FX_BK + core * 8;
+            const float* p = nullptr;
+            if (j < 4) {
+                const int n = n0 + (GATED ? r % OUT : r);
+                if (n < g.N) p = g.w + (size_t)(GATED && r >= OUT ? g.N + n : n) * g.ldw + k;
+            } else if (r < rows) {
+                p = g.a + (size_t)(m0 + r) * g.lda + k;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                x[j][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p == nullptr) continue;
+                if (k + 4 * h + 4 <= g.K) {
+                    x[j][h] = *reinterpret_cast<const float4*>(p + 4 * h);
+                } else {
+                    if (k + 4 * h < g.K) x[j][h].x = p[4 * h];
+                    if (k + 4 * h + 1 < g.K) x[j][h].y = p[4 * h + 1];
+                    if (k + 4 * h + 2 < g.K) x[j][h].z = p[4 * h + 2];
+                }
+            }
+        };
+        float left = 0.0f;                            // what the numbers leave: finite as long as they are
+        auto split = [&](int j, uint8_t* dst, int part_bytes) {
+            const float v[8] = {x[j][0].x, x[j][0].y, x[j][0].z, x[j][0].w, x[j][1].x, x[j][1].y, x[j][1].z, x[j][1].w};
+            uint32_t o[3][4];
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                uint32_t b[3][2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    b[0][u] = __float_as_uint(v[i + u]) & 0xffff0000u;
+                    const float r = v[i + u] - __uint_as_float(b[0][u]);
+                    left += r;
+                    b[1][u] = __float_as_uint(r) & 0xffff0000u;
+                    b[2][u] = __float_as_uint(r - __uint_as_float(b[1][u]));
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) o[q][i >> 1] = __byte_perm(b[q][0], b[q][1], 0x7632);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * part_bytes) = make_uint4(o[q][0], o[q][1], o[q][2], o[q][3]);
+        };
+        // weights are constants: the first ones are on their way before the preceding kernel has ended
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (steps > 0) load(j, 0);
+        pdl_wait_prior_grids();
+#pragma unroll
+        for (int j = 4; j < 8; ++j) if (steps > 0) load(j, 0);
+        for (int t = 0; t < steps; ++t) {
+            const int s = t & 1;
+            if (t >= 2 && !tc::wait_uniform(&empty[s], ((t >> 1) - 1) & 1, abort_flag)) break;
+            uint8_t* base = fx_smem + s * stage_bytes;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int r = row0 + (j & 3) * 32;
+                if (j < 4) split(j, base + core * fx_core_bytes(FX_BN) + r * 16, w_part);
+                else if (r < g.bm) split(j, base + 3 * w_part + core * fx_core_bytes(g.bm) + r * 16, a_part);
+                if (t + 1 < steps) load(j, t + 1);
+            }
+            // written through the generic proxy, read by the tensor core through the async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+        if (!(fabsf(left) < INFINITY)) odd_s[0] = 1.0f;
+    } else {
+        // -------------------------------------------------------- read-back --
+#pragma unroll
+        for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
+        const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int t = 0; t < steps; ++t) {
+            const int s = t & 1;
+            if (!tc::wait_uniform(&acc_full[s], (t >> 1) & 1, abort_flag)) break;
+            tc::tc_fence_after();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int c0 = (2 * i + (warp >> 2)) * 16;
+                if (c0 < g.bm) {                      // warp-uniform
+                    uint32_t d0[16], d1[16];
+                    tc::tmem_ld<16>(at + s * 256 + c0, d0);
+                    tc::tmem_ld<16>(at + s * 256 + 128 + c0, d1);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) acc[i * 16 + e] += __uint_as_float(d0[e]) + __uint_as_float(d1[e]);
+                }
+            }
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[s]);
+        }
+    }
+    __syncthreads();                                  // every MMA has run: the sums go where the stages were
+    float* sums = reinterpret_cast<float*>(fx_smem);  // [activation row][FX_LD]
+    if (warp < FX_READERS / 32) {
+        const int n = (warp & 3) * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c0 = (2 * i + (warp >> 2)) * 16;
+            if (c0 < g.bm) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) sums[(c0 + e) * FX_LD + n] = acc[i * 16 + e];
+            }
+        }
+    }
+    cluster_sync_all();
+    const float odd = cluster_sum4(odd_s, g.splits).x;
+    const int own = (rows + g.splits - 1) / g.splits;
+    for (int i = tid; i < own * (OUT / 4); i += FX_THREADS) {
+        const int r = i / (OUT / 4), col = (i - r * (OUT / 4)) * 4, m = rank * own + r;
+        if (m >= rows || n0 + col >= g.N) continue;
+        float v[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+        if (odd == 0.0f) {
+            const float4 x = cluster_sum4(sums + m * FX_LD + col, g.splits);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            if (GATED) {
+                const float4 z = cluster_sum4(sums + m * FX_LD + OUT + col, g.splits);
+                u[0] = z.x; u[1] = z.y; u[2] = z.z; u[3] = z.w;
+            }
+        } else {
+            const float* a = g.a + (size_t)(m0 + m) * g.lda;
+            for (int j = 0; j < 4 && n0 + col + j < g.N; ++j)
+                for (int k = 0; k < g.K; ++k) {
+                    v[j] = fmaf(a[k], g.w[(size_t)(n0 + col + j) * g.ldw + k], v[j]);
+                    if (GATED) u[j] = fmaf(a[k], g.w[(size_t)(g.N + n0 + col + j) * g.ldw + k], u[j]);
+                }
+        }
+        if (GATED) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = gelu_tanh(v[j]) * u[j];
+        }
+        tc_store4<TWM_EPI_STORE_F32>(g.c, (size_t)(m0 + m) * g.ldc, n0 + col, g.N, v);
+    }
+    cluster_sync_all();                               // nobody leaves while its sums may still be read
+    if (warp == FX_THREADS / 32 - 1) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem, 512);
+    }
+}
+
+}  // namespace dense
+}  // namespace twm

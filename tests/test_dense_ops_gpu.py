@@ -102,3 +102,40 @@ def test_gemm_few_tiles(m, n, k, lda, epi):
     if epi != _dense.EPI_STORE_F32:
         off = off + 2.0 ** -8 * ref.abs()
     assert bool(((got - ref).abs() <= off + 1e-30).all())
+
+
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
+@pytest.mark.parametrize("m,n,k", [(9, 65, 2048), (16, 2048, 8190), (80, 300, 64), (128, 1000, 72), (129, 64, 1000), (200, 129, 4100)])
+def test_gemm_f32_split_operands(m, n, k, epi):
+    """FP32 products as sums of bfloat16 products: numbers of very different size, no worse than FP32 sums; K in clusters and not."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rows, ld = (2 * n if epi == _dense.EPI_GELU_GLU else n), (k + 3) // 4 * 4
+    a = torch.zeros((m, ld), device="cuda")
+    w = torch.zeros((rows, ld), device="cuda")
+    a[:, :k] = torch.randn((m, k), generator=gen, device="cuda") * torch.exp(2 * torch.randn((m, k), generator=gen, device="cuda"))
+    w[:, :k] = torch.randn((rows, k), generator=gen, device="cuda") / math.sqrt(k)
+    got = gemm(a[:, :k], w[:, :k], epi, 0, n, ldc=n + 1)
+    # k + 16 roundings of at most 2^-24 of what has been added up (the products left out: 2^-21 of theirs at most)
+    ref, off = a[:, :k].double() @ w[:, :k].double().T, (a[:, :k].abs().double() @ w[:, :k].abs().double().T) * (k + 16) * 2.0 ** -24
+    if epi == _dense.EPI_GELU_GLU:
+        gate, up = ref[:, :n], ref[:, n:]
+        off = 1.2 * off[:, :n] * up.abs() + (gate.abs() + 1.2 * off[:, :n]) * off[:, n:] + 2.0 ** -20 * (gate * up).abs()
+        ref = gelu_tanh(gate) * up
+    assert bool(((got - ref).abs() <= off + 1e-30).all())
+
+
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan, 3.4e38])
+def test_gemm_f32_numbers_without_a_split(value):
+    """Infinities, NaN and the largest numbers come out as FP32 FMAs give them, in every row, also where K is shared by a cluster."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    m, n, k = 33, 200, 1024
+    a = torch.randn((m, k), generator=gen, device="cuda")
+    w = torch.randn((n, k), generator=gen, device="cuda") / 32
+    a[5, 700] = value
+    got = gemm(a, w, _dense.EPI_STORE_F32, 0, n)
+    ref = a.double() @ w.double().T
+    assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf())
+    fine = ref.isfinite()
+    assert torch.equal(got[~fine & ~ref.isnan()], ref[~fine & ~ref.isnan()])
+    off = (a.abs().double() @ w.abs().double().T) * (k + 16) * 2.0 ** -24
+    assert bool(((got - ref).abs() <= off)[fine].all())
