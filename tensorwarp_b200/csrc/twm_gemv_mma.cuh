@@ -517,6 +517,25 @@ gemv_kernel(const __grid_constant__ GemmParams p)
         // reaches the barrier (all loops above are bounded).
         const uint32_t rank = cluster_ctarank();
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // pairs with the arrive at the top: every CTA of the cluster runs
+        if (MP > CLUSTER_ROWS) {
+            // three to eight rows: each CTA leaves its sums where its weights were and adds up a share of the tile over the
+            // cluster, in slice order (four rows, N=4608, K=3584: 10.2 us through the workspace, 6.5 here; N=2048, K=2048: 10.9 and 4.7)
+            constexpr int LD = NT + 4;
+            float* sums = reinterpret_cast<float*>(&sm.packed[0][0]);
+            if (consumer) {
+                named_bar_sync(1, CONSUMERS);                            // every consumer warp has read its stages
+                float* to = sums + mA * LD + wcol + g;
+                to[0] = tot[0]; to[LD] = tot[1]; to[8] = tot[2]; to[LD + 8] = tot[3];
+            }
+            cluster_sync_all();
+            if (consumer && *abort_flag == 0)
+                for (int i = (int)rank * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
+                    const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+                    if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));
+                }
+            cluster_sync_all();                                          // nobody leaves while its sums may still be read
+            return;
+        }
         if (consumer && t == 0 && *abort_flag == 0) {
             const uint32_t base = mapa_shared(smem_u32(&sm.red[rank * p.M][0]), 0);
             st_cluster_f32(base + (wcol + g) * 4, tot[0]);

@@ -38,7 +38,7 @@ void set_error(const char* where, cudaError_t e)
 constexpr int kMaxDevices = 64;
 constexpr int kDefaultSms = 148;
 constexpr int kMaxSplits = 64;
-// K slices that add up as a cluster, at most: staged rows of the streaming kernel, and up to four rows of the FP32 kernel
+// K slices that add up as a cluster, at most: three rows or more of the streaming kernel, and up to four rows of the FP32 kernel
 constexpr int kMaxStagedSlices = 8, kMaxSimtSlices = 16;
 constexpr size_t kCounterBytes = 16384;   // 4096 tile counters at the head of the workspace
 
@@ -692,9 +692,9 @@ twm_status plan_impl(int M, int N, int K, int group_size, int sm_count, int spli
         bps = cluster_blocks(n_tiles * ((rows + twm::tcw::MB - 1) / twm::tcw::MB), nkb, sm_count, 0.8, 4.0);
         splits = (nkb + bps - 1) / bps;
     } else {
-        // The slices of staged rows and of up to four rows of the FP32 kernel are a cluster too, though room in the workspace is asked
+        // The slices of three rows or more and of up to four rows of the FP32 kernel are a cluster too, though room in the workspace is asked
         // for.  (Five to eight FP32 rows, one CTA to an SM: six slices of a cluster 44 us, eighteen through the workspace 31.)
-        const bool staged = kernel == TWM_KERNEL_MMA && prepass == 1 && mma_prepass(rows, K, N), simt = kernel == TWM_KERNEL_SIMT && mmax_for(rows) <= 4;
+        const bool staged = kernel == TWM_KERNEL_MMA && !can_cluster && prepass != 2, simt = kernel == TWM_KERNEL_SIMT && mmax_for(rows) <= 4;
         const int most = can_cluster ? twm::mma::MAX_CLUSTER / rows : staged ? kMaxStagedSlices : simt ? kMaxSimtSlices : kMaxSplits;
         choose_splits(n_tiles, nkb, slots, sm_count, max_bps, align, most, can_cluster || staged || simt, staged || simt, &splits, &bps);
         if (bps > max_bps) return TWM_EINVAL;
@@ -848,6 +848,7 @@ twm_status twm_gemm_w4a16(const twm_gemm_args* a, void* stream_)
         p.cluster_reduce = (pl.cluster_reduce && (kernel != TWM_KERNEL_MMA || rows <= twm::mma::CLUSTER_ROWS)) ? 1 : 0;
         const bool staged = kernel == TWM_KERNEL_MMA && prepass && rows >= (prepass == 2 ? 2 : 3);
         if (staged) p.cluster_reduce = pl.splits > 1 && pl.splits <= kMaxStagedSlices && !a->comm;
+        else if (kernel == TWM_KERNEL_MMA && rows > twm::mma::CLUSTER_ROWS) p.cluster_reduce = pl.splits > 1 && pl.splits <= kMaxStagedSlices && !a->comm;
         if (kernel == TWM_KERNEL_SIMT) p.cluster_reduce = pl.splits > 1 && pl.splits <= kMaxSimtSlices && mmax_for(a->M) <= 4;
         p.accumulate = (a->flags & TWM_FLAG_ACCUMULATE) ? 1 : 0;
         p.no_wait = ((a->flags & TWM_FLAG_INDEPENDENT) && (a->flags & TWM_FLAG_PDL) && kernel == TWM_KERNEL_MMA &&

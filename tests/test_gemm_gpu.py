@@ -724,9 +724,10 @@ def test_tensor_parallel_shard_shapes(k, n):
 
 @pytest.mark.parametrize("m,k,n,group,splits,f32", [(1, 512, 130, 32, 16, True), (2, 608, 64, 32, 7, True), (4, 4096, 300, 128, 0, True), (3, 1024, 129, 128, 9, True),
                                                     (5, 1024, 200, 32, 3, True), (1, 544, 40, 32, 17, True), (9, 1024, 300, 32, 8, False), (24, 1152, 129, 128, 9, False),
-                                                    (31, 2048, 258, 128, 0, False)])
+                                                    (31, 2048, 258, 128, 0, False), (3, 1024, 300, 128, 8, False), (5, 2048, 129, 32, 0, False),
+                                                    (8, 1152, 130, 128, 9, False), (8, 3584, 40, 128, 7, False)])
 def test_few_rows_in_slices(m, k, n, group, splits, f32):
-    """K slices that are a cluster (FP32 rows up to four, staged rows up to eight slices) and those that are not: ragged
+    """K slices that are a cluster (FP32 rows up to four; three rows or more of the streaming kernel up to eight slices) and those that are not: ragged
     columns, the accumulate flag, rows of C off 16 bytes, and the same bits every time."""
     kern, dt = (_lib.TWM_KERNEL_SIMT, torch.float32) if f32 else (_lib.TWM_KERNEL_MMA, torch.float16)
     _, packed, scales = _quantised(k, n, group, 67)
