@@ -1,8 +1,10 @@
 // twm_dense_f32tc.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models on the tensor cores, with the error of an FP32 product.
 //
-// Every FP32 number is exactly the sum of three bfloat16 numbers: its leading eight bits, the next eight, the last eight (cut, so
-// that all have its sign).  A product of two is the sum of nine; the six largest are taken, the others are below 2^-21 of it
-// (2^-24 on average).  The tensor core multiplies them exactly, but cuts when it adds.  So the products of the leading parts (acc 0)
+// An FP32 number is the sum of three bfloat16 numbers: its leading eight bits, the next eight, the last eight (cut, so that all
+// have its sign).  The last of them lies up to 2^-23 below the number, so operands are multiplied by 2^24 first and the sums by 2^-48
+// at the end, both exactly: below 2^-110 the parts would run into bfloat16's smallest number (2^-133) and be cut (activations of
+// 2^-120, K = 1024: errors of 1.6e-5 of the sum of absolute products without the factor, 3.7e-8 with it, 2.4e-7 in FP32 FMAs).
+// A product of two is the sum of nine; the six largest are taken, the others are below 2^-21 of it (2^-24 on average).  The tensor core multiplies them exactly, but cuts when it adds.  So the products of the leading parts (acc 0)
 // and the other five (acc 1, 2^-7 smaller) have accumulators of their own, and both are taken out and added up in FP32
 // registers every 64 K.
 //
@@ -11,8 +13,9 @@
 // 8-15 read FP32 rows from global memory, split them and write the six operands to shared memory, 16 issues the MMAs.  A stage moves
 // 160 KB through shared memory at 80 rows (24 MMAs read 6.5 KB each), which is what bounds it.
 //
-// A number that is not finite has no such sum.  The splitting threads notice one (what a number leaves behind its leading
-// part is then not a number), and the cluster computes its tile with plain FP32 FMAs instead.
+// A number that is not finite, or not below 2^104, has no such sum.  The splitting threads notice one (what a number leaves behind
+// its leading part is then not a number), the reading threads a sum that has outgrown FP32 (from 2^80 on with the factors), and the
+// cluster computes its tile with plain FP32 FMAs instead.
 #pragma once
 
 #include "twm_dense_f32.cuh"
@@ -28,6 +31,8 @@ __host__ __device__ constexpr int fx_core_bytes(int rows) { return rows * 16 + 1
 __host__ __device__ constexpr int fx_part_bytes(int rows) { return FX_CORES * fx_core_bytes(rows); }
 __host__ __device__ constexpr int fx_stage_bytes(int bm) { return 3 * (fx_part_bytes(FX_BN) + fx_part_bytes(bm)); }
 inline size_t fx_smem_bytes(int bm) { return std::max(2 * fx_stage_bytes(bm), bm * FX_LD * 4) + 128; }
+
+constexpr float FX_SCALE = 16777216.0f, FX_UNSCALE = 1.0f / (FX_SCALE * FX_SCALE);     // 2^24 and 2^-48
 
 struct GemmFxArgs {
     const float *a, *w;
@@ -46,7 +51,7 @@ gemm_f32tc_kernel(const GemmFxArgs g)
     __shared__ __align__(8) uint64_t full[2], empty[2], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_s;
     __shared__ int abort_s;
-    __shared__ __align__(16) float odd_s[4];         // [0]: not zero where a number was not finite
+    __shared__ __align__(16) float odd_s[4];         // [0]: not zero where a number has no split or a sum is not finite
     volatile int* abort_flag = &abort_s;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -145,8 +150,9 @@ gemm_f32tc_kernel(const GemmFxArgs g)
                 uint32_t b[3][2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    b[0][u] = __float_as_uint(v[i + u]) & 0xffff0000u;
-                    const float r = v[i + u] - __uint_as_float(b[0][u]);
+                    const float f = v[i + u] * FX_SCALE;
+                    b[0][u] = __float_as_uint(f) & 0xffff0000u;
+                    const float r = f - __uint_as_float(b[0][u]);
                     left += r;
                     b[1][u] = __float_as_uint(r) & 0xffff0000u;
                     b[2][u] = __float_as_uint(r - __uint_as_float(b[1][u]));
@@ -205,6 +211,10 @@ gemm_f32tc_kernel(const GemmFxArgs g)
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[s]);
         }
+        bool fine = true;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) fine = fine && fabsf(acc[i]) < INFINITY;
+        if (!fine) odd_s[0] = 1.0f;
     }
     __syncthreads();                                  // every MMA has run: the sums go where the stages were
     float* sums = reinterpret_cast<float*>(fx_smem);  // [activation row][FX_LD]
@@ -228,10 +238,10 @@ gemm_f32tc_kernel(const GemmFxArgs g)
         float v[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
         if (odd == 0.0f) {
             const float4 x = cluster_sum4(sums + m * FX_LD + col, g.splits);
-            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            v[0] = x.x * FX_UNSCALE; v[1] = x.y * FX_UNSCALE; v[2] = x.z * FX_UNSCALE; v[3] = x.w * FX_UNSCALE;
             if (GATED) {
                 const float4 z = cluster_sum4(sums + m * FX_LD + OUT + col, g.splits);
-                u[0] = z.x; u[1] = z.y; u[2] = z.z; u[3] = z.w;
+                u[0] = z.x * FX_UNSCALE; u[1] = z.y * FX_UNSCALE; u[2] = z.z * FX_UNSCALE; u[3] = z.w * FX_UNSCALE;
             }
         } else {
             const float* a = g.a + (size_t)(m0 + m) * g.lda;

@@ -139,3 +139,15 @@ def test_gemm_f32_numbers_without_a_split(value):
     assert torch.equal(got[~fine & ~ref.isnan()], ref[~fine & ~ref.isnan()])
     off = (a.abs().double() @ w.abs().double().T) * (k + 16) * 2.0 ** -24
     assert bool(((got - ref).abs() <= off)[fine].all())
+
+
+@pytest.mark.parametrize("k", [64, 1024, 8192])
+@pytest.mark.parametrize("sa,sw", [(-120, 0), (-125, 0), (-140, 20), (0, -126), (-70, -70), (60, 40), (110, 0), (126, -100)])
+def test_gemm_f32_small_and_large_numbers(sa, sw, k):
+    """Operands whose last bits lie below bfloat16's smallest number, or that leave no room above: as good as in the middle of the range."""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    a, w = (torch.randn((r, k), generator=gen, device="cuda", dtype=torch.float64).clamp(-3.9, 3.9).mul(2.0 ** s).float() for r, s in ((70, sa), (300, sw)))
+    got = gemm(a, w, _dense.EPI_STORE_F32, 0, 300)
+    # products left out: 2^-21 of theirs at most; then a rounding of 2^-24 for every 64 K and every CTA of a cluster, and of the result
+    ref, off = a.double() @ w.double().T, (a.double().abs() @ w.double().abs().T) * (k / 64 + 8 + 8 + 1) * 2.0 ** -24 + 2.0 ** -149
+    assert bool(((got - ref).abs() <= off).all())
