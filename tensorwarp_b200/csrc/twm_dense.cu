@@ -485,7 +485,10 @@ twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, i
 // From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 5 rows 2.37 / 2.72,
 // 9 rows 2.80 / 2.75, 20 rows 3.33 / 2.84, 70 rows 6.45 / 3.51, 256 rows 18.2 / 8.1; error against 64 bits of 70 rows x 2048 x 8192:
 // 4.1e-7 / 1.5e-7.
-constexpr int F32TC_ROWS = 9;
+// Error against 64 bits over the sum of absolute products (largest, RMS), 70 rows, FP32 FMAs / tensor cores: K = 1 6.0e-8, 2.5e-8 / 8.9e-8,
+// 2.6e-8; K = 2 1.1e-7, 2.6e-8 / 1.5e-7, 2.2e-8; K = 8 1.9e-7, 2.7e-8 / 1.3e-7, 1.5e-8; K = 1024 2.4e-7, 2.8e-8 / 2.7e-8, 4.6e-9: sums of
+// fewer than eight products stay on the plain tiles.
+constexpr int F32TC_ROWS = 9, F32TC_K = 8;
 
 // K over as many CTAs of a cluster as cost least, counted in stages of 64 K (about 1 us): waves of the clusters that run at once, and
 // four stages' time for the exchange of the sums.
@@ -533,7 +536,7 @@ twm_status gemm(const T* a, int lda, const T* w, int ldw, void* c, int ldc, int 
     if (kernel >= 2 && !fits) return invalid("the tcgen05 product takes bfloat16 rows on 16-byte boundaries");
     if (kernel >= 2 || (kernel == 0 && fits))
         return gemm_tc_any(a, lda, w, ldw, c, ldc, M, N, K, epi, kernel > 2 ? kernel : 0, flags, stream);
-    if (f32_fits(a, lda, w, ldw) && (epi == TWM_EPI_STORE || epi == TWM_EPI_STORE_F32 || epi == TWM_EPI_GELU_GLU))
+    if (f32_fits(a, lda, w, ldw) && (M < F32TC_ROWS || K >= F32TC_K) && (epi == TWM_EPI_STORE || epi == TWM_EPI_STORE_F32 || epi == TWM_EPI_GELU_GLU))
         return gemm_f32_any(a, lda, w, ldw, c, ldc, M, N, K, epi, flags, stream);
     const dim3 grid((N + ST - 1) / ST, (M + ST - 1) / ST);
     switch (epi) {

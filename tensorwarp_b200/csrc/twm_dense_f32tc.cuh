@@ -1,11 +1,12 @@
 // twm_dense_f32tc.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models on the tensor cores, with the error of an FP32 product.
 //
-// An FP32 number is the sum of three bfloat16 numbers: its leading eight bits, the next eight, the last eight (cut, so that all
-// have its sign).  The last of them lies up to 2^-23 below the number, so operands are multiplied by 2^24 first and the sums by 2^-48
-// at the end, both exactly: below 2^-110 the parts would run into bfloat16's smallest number (2^-133) and be cut (activations of
-// 2^-120, K = 1024: errors of 1.6e-5 of the sum of absolute products without the factor, 3.7e-8 with it, 2.4e-7 in FP32 FMAs).
-// A product of two is the sum of nine; the six largest are taken, the others are below 2^-21 of it (2^-24 on average).  The tensor core multiplies them exactly, but cuts when it adds.  So the products of the leading parts (acc 0)
-// and the other five (acc 1, 2^-7 smaller) have accumulators of their own, and both are taken out and added up in FP32
+// An FP32 number is the sum of three bfloat16 numbers: itself rounded to the nearest, what that leaves rounded to the nearest, and the
+// rest (23 bits and two signs: nothing is left).  The last of them lies up to 2^-23 below the number, so operands are multiplied by 2^24
+// first and the sums by 2^-48 at the end, both exactly: below 2^-110 the parts would run into bfloat16's smallest number (2^-133) and
+// be cut (activations of 2^-120, K = 1024: errors of 1.6e-5 of the sum of absolute products without the factor, 2.7e-8 with it, 2.4e-7
+// in FP32 FMAs).  A product of two is the sum of nine; the six largest are taken, the others are below 2^-24 of it, which is
+// what an FP32 product rounds by (cut instead of rounded parts: 2^-21).  The tensor core multiplies them exactly, but cuts when it adds.  So the products of the leading parts (acc 0)
+// and the other five (acc 1, 2^-8 smaller) have accumulators of their own, and both are taken out and added up in FP32
 // registers every 64 K.
 //
 // Tile: 128 weight rows (the MMA's M) x up to 128 activation rows, 64 K a stage, two stages, one CTA to an SM, K shared by a
@@ -13,9 +14,9 @@
 // 8-15 read FP32 rows from global memory, split them and write the six operands to shared memory, 16 issues the MMAs.  A stage moves
 // 160 KB through shared memory at 80 rows (24 MMAs read 6.5 KB each), which is what bounds it.
 //
-// A number that is not finite, or not below 2^104, has no such sum.  The splitting threads notice one (what a number leaves behind
-// its leading part is then not a number), the reading threads a sum that has outgrown FP32 (from 2^80 on with the factors), and the
-// cluster computes its tile with plain FP32 FMAs instead.
+// A number that is not finite, or not below 2^104, has no such sum: its second part is not a number, nor is any sum that it enters.  The
+// reading threads notice that, or a sum that has outgrown FP32 (from 2^80 on with the factors), and the cluster computes its tile
+// with plain FP32 FMAs instead.
 #pragma once
 
 #include "twm_dense_f32.cuh"
@@ -141,24 +142,20 @@ gemm_f32tc_kernel(const GemmFxArgs g)
                 }
             }
         };
-        float left = 0.0f;                            // what the numbers leave: finite as long as they are
         auto split = [&](int j, uint8_t* dst, int part_bytes) {
             const float v[8] = {x[j][0].x, x[j][0].y, x[j][0].z, x[j][0].w, x[j][1].x, x[j][1].y, x[j][1].z, x[j][1].w};
             uint32_t o[3][4];
 #pragma unroll
             for (int i = 0; i < 8; i += 2) {
-                uint32_t b[3][2];
+                float f[2] = {v[i] * FX_SCALE, v[i + 1] * FX_SCALE};
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const float f = v[i + u] * FX_SCALE;
-                    b[0][u] = __float_as_uint(f) & 0xffff0000u;
-                    const float r = f - __uint_as_float(b[0][u]);
-                    left += r;
-                    b[1][u] = __float_as_uint(r) & 0xffff0000u;
-                    b[2][u] = __float_as_uint(r - __uint_as_float(b[1][u]));
+                for (int q = 0; q < 3; ++q) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(f[0], f[1]);
+                    o[q][i >> 1] = *reinterpret_cast<const uint32_t*>(&b);
+                    if (q == 2) break;
+                    f[0] -= __uint_as_float(o[q][i >> 1] << 16);
+                    f[1] -= __uint_as_float(o[q][i >> 1] & 0xffff0000u);
                 }
-#pragma unroll
-                for (int q = 0; q < 3; ++q) o[q][i >> 1] = __byte_perm(b[q][0], b[q][1], 0x7632);
             }
 #pragma unroll
             for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * part_bytes) = make_uint4(o[q][0], o[q][1], o[q][2], o[q][3]);
@@ -185,7 +182,6 @@ gemm_f32tc_kernel(const GemmFxArgs g)
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
         }
-        if (!(fabsf(left) < INFINITY)) odd_s[0] = 1.0f;
     } else {
         // -------------------------------------------------------- read-back --
 #pragma unroll

@@ -148,6 +148,26 @@ def test_gemm_f32_small_and_large_numbers(sa, sw, k):
     gen = torch.Generator(device="cuda").manual_seed(k)
     a, w = (torch.randn((r, k), generator=gen, device="cuda", dtype=torch.float64).clamp(-3.9, 3.9).mul(2.0 ** s).float() for r, s in ((70, sa), (300, sw)))
     got = gemm(a, w, _dense.EPI_STORE_F32, 0, 300)
-    # products left out: 2^-21 of theirs at most; then a rounding of 2^-24 for every 64 K and every CTA of a cluster, and of the result
-    ref, off = a.double() @ w.double().T, (a.double().abs() @ w.double().abs().T) * (k / 64 + 8 + 8 + 1) * 2.0 ** -24 + 2.0 ** -149
+    # products left out: 2^-24 of theirs at most; then a rounding of 2^-24 for every 64 K and every CTA of a cluster, and two of the result
+    ref, off = a.double() @ w.double().T, (a.double().abs() @ w.double().abs().T) * (1 + k / 64 + 8 + 2) * 2.0 ** -24 + 2.0 ** -149
     assert bool(((got - ref).abs() <= off).all())
+
+
+@pytest.mark.parametrize("m", [9, 70])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 7, 8, 12, 16])
+def test_gemm_f32_few_products(m, k):
+    """Sums of a few products are as good as FP32 FMAs: a rounding of 2^-24 each."""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    a, w = (torch.randn((r, 16), generator=gen, device="cuda")[:, :k] for r in (m, 500))
+    got = gemm(a, w, _dense.EPI_STORE_F32, 0, 500)
+    ref, off = a.double() @ w.double().T, (a.double().abs() @ w.double().abs().T) * k * 2.0 ** -24
+    assert bool(((got - ref).abs() <= off).all())
+
+
+def test_gemm_f32_lone_products():
+    """One product in a sum of zeros: the products left out and the two roundings of the sum are 2^-24 of it at most each."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, w = torch.zeros((70, 1024), device="cuda"), torch.randn((500, 1024), generator=gen, device="cuda")
+    a[:, 500] = torch.randn(70, generator=gen, device="cuda")
+    got, ref = gemm(a, w, _dense.EPI_STORE_F32, 0, 500), a.double() @ w.double().T
+    assert bool(((got - ref).abs() <= 3 * 2.0 ** -24 * ref.abs()).all())
