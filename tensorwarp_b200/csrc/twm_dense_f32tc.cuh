@@ -42,6 +42,49 @@ struct GemmFxArgs {
     int m_tiles, bm, splits;        // bm: activation rows a tile, a multiple of 16
 };
 
+// Rows first ... (count of them) of a tile with FP32 FMAs: a warp takes two rows x four weight rows, its lanes along K.  70 rows, 2048 x
+// 8192, one NaN: 6 714 us with a thread along K for each four results, 330 us this way (the plain tiles of twm_dense_simt.cuh: 573); 1024 rows: 71 204 and 3 031.
+template <int EPI>
+__device__ __forceinline__ void fx_plain(const GemmFxArgs g, int first, int count, int n0)
+{
+    constexpr bool GATED = EPI == TWM_EPI_GELU_GLU;
+    constexpr int COLS = GATED ? 2 : 4, ITEMS = FX_BN / 4;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int i = threadIdx.x >> 5; i < (count + 1) / 2 * ITEMS; i += FX_THREADS / 32) {
+        const int m = first + i / ITEMS * 2, n = n0 + i % ITEMS * COLS;
+        if (n >= g.N) continue;
+        const float *a0 = g.a + (size_t)m * g.lda, *a1 = a0 + (m + 1 < first + count ? g.lda : 0), *w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = g.w + (size_t)(min(n + j % COLS, g.N - 1) + (GATED && j >= COLS ? g.N : 0)) * g.ldw;
+        float s[8] = {};
+#pragma unroll 2
+        for (int k = lane * 4; k < g.K; k += 128) {
+            auto four = [&](const float* p) {
+                if (k + 4 <= g.K) return *reinterpret_cast<const float4*>(p + k);
+                return make_float4(p[k], k + 1 < g.K ? p[k + 1] : 0.f, k + 2 < g.K ? p[k + 2] : 0.f, 0.f);
+            };
+            const float4 x = four(a0), y = four(a1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 v = four(w[j]);
+                s[j] = fmaf(x.w, v.w, fmaf(x.z, v.z, fmaf(x.y, v.y, fmaf(x.x, v.x, s[j]))));
+                s[4 + j] = fmaf(y.w, v.w, fmaf(y.z, v.z, fmaf(y.y, v.y, fmaf(y.x, v.x, s[4 + j]))));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] = ops::warp_sum(s[j]);
+        if (lane == 0) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int j = 0; j < COLS; ++j)
+                    if (m + r < first + count && n + j < g.N)
+                        g.c[(size_t)(m + r) * g.ldc + n + j] = GATED ? gelu_tanh(s[4 * r + j]) * s[4 * r + 2 + j] : s[4 * r + j];
+        }
+    }
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(FX_THREADS, 1)
 gemm_f32tc_kernel(const GemmFxArgs g)
@@ -226,32 +269,23 @@ gemm_f32tc_kernel(const GemmFxArgs g)
         }
     }
     cluster_sync_all();
-    const float odd = cluster_sum4(odd_s, g.splits).x;
-    const int own = (rows + g.splits - 1) / g.splits;
-    for (int i = tid; i < own * (OUT / 4); i += FX_THREADS) {
-        const int r = i / (OUT / 4), col = (i - r * (OUT / 4)) * 4, m = rank * own + r;
-        if (m >= rows || n0 + col >= g.N) continue;
-        float v[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
-        if (odd == 0.0f) {
+    const int own = (rows + g.splits - 1) / g.splits, first = rank * own;
+    if (cluster_sum4(odd_s, g.splits).x != 0.0f) {    // the same in every CTA: nobody reads the sums
+        fx_plain<EPI>(g, m0 + first, min(own, rows - first), n0);
+    } else {
+        for (int i = tid; i < own * (OUT / 4); i += FX_THREADS) {
+            const int r = i / (OUT / 4), col = (i - r * (OUT / 4)) * 4, m = first + r;
+            if (m >= rows || n0 + col >= g.N) continue;
             const float4 x = cluster_sum4(sums + m * FX_LD + col, g.splits);
-            v[0] = x.x * FX_UNSCALE; v[1] = x.y * FX_UNSCALE; v[2] = x.z * FX_UNSCALE; v[3] = x.w * FX_UNSCALE;
+            float v[4] = {x.x * FX_UNSCALE, x.y * FX_UNSCALE, x.z * FX_UNSCALE, x.w * FX_UNSCALE};
             if (GATED) {
                 const float4 z = cluster_sum4(sums + m * FX_LD + OUT + col, g.splits);
-                u[0] = z.x * FX_UNSCALE; u[1] = z.y * FX_UNSCALE; u[2] = z.z * FX_UNSCALE; u[3] = z.w * FX_UNSCALE;
-            }
-        } else {
-            const float* a = g.a + (size_t)(m0 + m) * g.lda;
-            for (int j = 0; j < 4 && n0 + col + j < g.N; ++j)
-                for (int k = 0; k < g.K; ++k) {
-                    v[j] = fmaf(a[k], g.w[(size_t)(n0 + col + j) * g.ldw + k], v[j]);
-                    if (GATED) u[j] = fmaf(a[k], g.w[(size_t)(g.N + n0 + col + j) * g.ldw + k], u[j]);
-                }
-        }
-        if (GATED) {
+                const float u[4] = {z.x * FX_UNSCALE, z.y * FX_UNSCALE, z.z * FX_UNSCALE, z.w * FX_UNSCALE};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = gelu_tanh(v[j]) * u[j];
+                for (int j = 0; j < 4; ++j) v[j] = gelu_tanh(v[j]) * u[j];
+            }
+            tc_store4<TWM_EPI_STORE_F32>(g.c, (size_t)(m0 + m) * g.ldc, n0 + col, g.N, v);
         }
-        tc_store4<TWM_EPI_STORE_F32>(g.c, (size_t)(m0 + m) * g.ldc, n0 + col, g.N, v);
     }
     cluster_sync_all();                               // nobody leaves while its sums may still be read
     if (warp == FX_THREADS / 32 - 1) {

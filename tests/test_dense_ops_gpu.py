@@ -171,3 +171,43 @@ def test_gemm_f32_lone_products():
     a[:, 500] = torch.randn(70, generator=gen, device="cuda")
     got, ref = gemm(a, w, _dense.EPI_STORE_F32, 0, 500), a.double() @ w.double().T
     assert bool(((got - ref).abs() <= 3 * 2.0 ** -24 * ref.abs()).all())
+
+
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
+@pytest.mark.parametrize("m,n,k", [(9, 65, 8), (17, 129, 1000), (70, 300, 2050), (128, 40, 96), (200, 130, 260)])
+def test_gemm_f32_tiles_without_a_split(m, n, k, epi):
+    """Tiles that hold an infinity or NaN, edges of rows, columns and K: the other numbers are those of FP32 FMAs, a tile without one is untouched."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rows, ld = (2 * n if epi == _dense.EPI_GELU_GLU else n), (k + 3) // 4 * 4
+    a, w = torch.full((m, ld), 1e30, device="cuda")[:, :k], torch.full((rows, ld), 1e30, device="cuda")[:, :k]
+    a.copy_(torch.randn((m, k), generator=gen, device="cuda"))
+    w.copy_(torch.randn((rows, k), generator=gen, device="cuda") / math.sqrt(k))
+    fine = gemm(a, w, epi, 0, n, ldc=n + 3)
+    a[m - 1, k - 1], w[n - 1, 0] = math.nan, math.inf
+    got, ref = gemm(a, w, epi, 0, n, ldc=n + 3), a.double() @ w.double().T
+    off = (a.abs().double() @ w.abs().double().T) * (k + 16) * 2.0 ** -24
+    if epi == _dense.EPI_GELU_GLU:
+        gate, up = ref[:, :n], ref[:, n:]
+        # |gelu'| < 1.2; tanh and the two products round by 2^-20 of a value of at most |gate|
+        off = 1.2 * off[:, :n] * up.abs() + (gate.abs() + 1.2 * off[:, :n]) * off[:, n:] + 2.0 ** -20 * (gate * up).abs()
+        ref = gelu_tanh(gate) * up
+    assert bool(((got - ref).abs() <= off + 1e-30)[:-1, :-1].all())
+    assert bool(got[-1].isnan().all()) and not bool(got[:-1, -1].isfinite().any() if epi == _dense.EPI_STORE_F32 else False)
+    assert bool(((got - fine).abs() <= 2 * off + 1e-30)[:-1, :-1].all())
+
+
+def test_gemm_f32_tiles_without_a_split_are_not_slow():
+    """One NaN costs no more than the plain tiles (which rows off 16-byte boundaries take)."""
+    a, w = torch.randn((70, 8192), device="cuda"), torch.randn((2048, 8193), device="cuda")
+    a[30, 4000] = math.nan
+
+    def timed(w):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        gemm(a, w, _dense.EPI_STORE_F32, 0, 2048)
+        start.record()
+        for _ in range(5):
+            gemm(a, w, _dense.EPI_STORE_F32, 0, 2048)
+        end.record()
+        torch.cuda.synchronize()
+        return start.elapsed_time(end)
+    assert timed(w[:, :8192].contiguous()) < 2 * timed(w[:, :8192])
