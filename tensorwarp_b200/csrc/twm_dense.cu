@@ -71,6 +71,25 @@ twm_status device(int* sms)
     return st.status;
 }
 
+// Lets the kernel take `smem` bytes of dynamic shared memory on the current device.  The limit belongs to the function and not to
+// a launch: it only grows, so that no thread lowers it between another's call of this and its launch.
+twm_status allow_smem(const char* what, const void* kernel, size_t smem)
+{
+    if (smem <= 32 * 1024) return TWM_OK;                // 48 KB without asking, static shared memory included
+    static std::unordered_map<const void*, size_t> allowed[64];
+    static std::mutex mutex;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return fail("cudaGetDevice", e);
+    if (dev < 0 || dev >= 64) return invalid("device index");
+    std::lock_guard<std::mutex> lock(mutex);
+    size_t& limit = allowed[dev][kernel];
+    if (smem <= limit) return TWM_OK;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return fail(what, e);
+    limit = smem;
+    return TWM_OK;
+}
+
 // One launch: raises the kernel's dynamic shared memory limit when needed, asks for programmatic dependent launch
 // when the caller allows it, and a cluster of `cluster` CTAs along x when > 0.
 template <typename... KArgs, typename... Args>
@@ -78,10 +97,7 @@ twm_status launch(const char* what, void (*kernel)(KArgs...), dim3 grid, int thr
                   int cluster, Args&&... args)
 {
     if (smem > kSmemLimit) return invalid("a row does not fit shared memory");
-    if (smem > 32 * 1024) {                              // 48 KB without asking, static shared memory included
-        const cudaError_t r = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (r != cudaSuccess) return fail(what, r);
-    }
+    TRY(allow_smem(what, (const void*)kernel, smem));
     if (cluster > 8) {
         const cudaError_t r = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (r != cudaSuccess) return fail(what, r);
@@ -354,7 +370,7 @@ twm_status cluster_capacity(int splits, int* out)
     if (n == 0) {
         auto kernel = gemm_tcs_kernel<128, TWM_EPI_STORE>;
         const int smem = 200 * 1024;
-        if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return fail("gemm_tcs", e);
+        TRY(allow_smem("gemm_tcs", (const void*)kernel, smem));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(splits);
         cfg.blockDim = dim3(TC_THREADS);

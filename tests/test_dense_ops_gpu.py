@@ -1,5 +1,7 @@
 """GPU tests of the single operations of the dense-weight decoders against plain PyTorch in float64."""
 import math
+import os
+import subprocess
 
 import pytest
 import torch
@@ -211,3 +213,16 @@ def test_gemm_f32_tiles_without_a_split_are_not_slow():
         torch.cuda.synchronize()
         return start.elapsed_time(end)
     assert timed(w[:, :8192].contiguous()) < 2 * timed(w[:, :8192])
+
+
+def test_products_from_two_threads(tmp_path):
+    """What a kernel may take of shared memory belongs to the function: threads whose products need different amounts of it are not refused."""
+    root, cuda = os.path.dirname(os.path.dirname(os.path.abspath(__file__))), os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    exe, lib = str(tmp_path / "two_threads"), os.path.join(root, "tensorwarp_b200")
+    _dense.lib()
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(root, "include"), "-I", os.path.join(cuda, "include"),
+                        os.path.join(root, "tests", "cpp", "two_threads.cpp"), "-o", exe, "-L", lib, "-ltwmdense", "-L", os.path.join(cuda, "lib64"), "-lcudart",
+                        "-lpthread", f"-Wl,-rpath,{lib}"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
