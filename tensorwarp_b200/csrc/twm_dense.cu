@@ -552,7 +552,7 @@ twm_status gemm(const T* a, int lda, const T* w, int ldw, void* c, int ldc, int 
     if (kernel >= 2 && !fits) return invalid("the tcgen05 product takes bfloat16 rows on 16-byte boundaries");
     if (kernel >= 2 || (kernel == 0 && fits))
         return gemm_tc_any(a, lda, w, ldw, c, ldc, M, N, K, epi, kernel > 2 ? kernel : 0, flags, stream);
-    if (f32_fits(a, lda, w, ldw) && (M < F32TC_ROWS || K >= F32TC_K) && (epi == TWM_EPI_STORE || epi == TWM_EPI_STORE_F32 || epi == TWM_EPI_GELU_GLU))
+    if (kernel == 0 && f32_fits(a, lda, w, ldw) && (M < F32TC_ROWS || K >= F32TC_K) && (epi == TWM_EPI_STORE || epi == TWM_EPI_STORE_F32 || epi == TWM_EPI_GELU_GLU))
         return gemm_f32_any(a, lda, w, ldw, c, ldc, M, N, K, epi, flags, stream);
     const dim3 grid((N + ST - 1) / ST, (M + ST - 1) / ST);
     switch (epi) {

@@ -33,8 +33,8 @@ def gelu_tanh(z):
 @pytest.mark.parametrize("m,n,k", [(1, 8, 16), (2, 48, 64), (5, 100, 80), (63, 130, 208), (128, 256, 512), (129, 257, 1040),
                                    (300, 1000, 336), (700, 2064, 128), (1024, 4096, 1024), (2100, 1530, 640)])
 @pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
-@pytest.mark.parametrize("dtype,kernel", [(torch.float32, 1), (torch.bfloat16, 1), (torch.bfloat16, 2), (torch.bfloat16, 64),
-                                          (torch.bfloat16, 128), (torch.bfloat16, 256), (torch.bfloat16, 512)])
+@pytest.mark.parametrize("dtype,kernel", [(torch.float32, 0), (torch.float32, 1), (torch.bfloat16, 0), (torch.bfloat16, 1), (torch.bfloat16, 2),
+                                          (torch.bfloat16, 64), (torch.bfloat16, 128), (torch.bfloat16, 256), (torch.bfloat16, 512)])
 def test_gemm(m, n, k, epi, dtype, kernel):
     gen = torch.Generator(device="cuda").manual_seed(m * 7 + n)
     a = torch.randn((m, k), generator=gen, device="cuda").to(dtype)
@@ -49,7 +49,7 @@ def test_gemm(m, n, k, epi, dtype, kernel):
 
 def test_gemm_rows_with_longer_strides_and_no_bleed():
     """Operands inside wider buffers: what lies past K, past M and past N must not enter the result."""
-    for dtype, kernel in ((torch.float32, 1), (torch.bfloat16, 1), (torch.bfloat16, 2)):
+    for dtype, kernel in ((torch.float32, 0), (torch.float32, 1), (torch.bfloat16, 0), (torch.bfloat16, 1), (torch.bfloat16, 2)):
         a = torch.full((200, 96), 1e30, device="cuda").to(dtype)
         w = torch.full((90, 112), 1e30, device="cuda").to(dtype)
         a[:70, :80] = torch.randn((70, 80), device="cuda").to(dtype)
@@ -57,6 +57,14 @@ def test_gemm_rows_with_longer_strides_and_no_bleed():
         got = gemm(a[:70, :80], w[:66, :80], _dense.EPI_STORE_F32, kernel, 66)
         ref = a[:70, :80].double() @ w[:66, :80].double().T
         assert float((got - ref).abs().max()) < 1e-3
+
+
+def test_gemm_f32_plain_tiles_when_asked():
+    """Kernel 1 is the plain tiles wherever the rows lie: the same bits on 16-byte boundaries and off them."""
+    for m in (5, 70):
+        a, w = torch.randn((m, 260), device="cuda"), torch.randn((90, 260), device="cuda")
+        off = [torch.empty((t.shape[0], 261), device="cuda")[:, :260].copy_(t) for t in (a, w)]
+        assert torch.equal(gemm(a, w, _dense.EPI_STORE_F32, 1, 90), gemm(*off, _dense.EPI_STORE_F32, 1, 90))
 
 
 @pytest.mark.parametrize("m,n,k,lda,ldw", [(1, 1, 1, 4, 4), (8, 127, 33, 36, 40), (9, 129, 2050, 2052, 2052), (64, 128, 32, 32, 32), (65, 1, 5000, 5000, 5000),
