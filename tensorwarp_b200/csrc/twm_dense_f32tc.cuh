@@ -121,6 +121,7 @@ gemm_f32tc_kernel(const GemmFxArgs g)
     __syncthreads();
     tc::tc_fence_after();
     pdl_launch_dependents();
+    cluster_started();
     const uint32_t tmem = tmem_s;
     float acc[64];                                    // readers: sums of chunks 2 i + (warp >> 2)
 
@@ -268,9 +269,11 @@ gemm_f32tc_kernel(const GemmFxArgs g)
             }
         }
     }
-    cluster_sync_all();
+    const bool all_ok = cluster_meet(abort_flag);
     const int own = (rows + g.splits - 1) / g.splits, first = rank * own;
-    if (cluster_sum4(odd_s, g.splits).x != 0.0f) {    // the same in every CTA: nobody reads the sums
+    if (!all_ok) {
+        // a wait ran out: nothing is stored, the error word is set
+    } else if (cluster_sum4(odd_s, g.splits).x != 0.0f) {    // the same in every CTA: nobody reads the sums
         fx_plain<EPI>(g, m0 + first, min(own, rows - first), n0);
     } else {
         for (int i = tid; i < own * (OUT / 4); i += FX_THREADS) {

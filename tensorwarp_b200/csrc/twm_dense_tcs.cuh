@@ -98,7 +98,9 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
     __syncthreads();
     tc::tc_fence_after();
     pdl_launch_dependents();
+    if (g.splits > 1) cluster_started();
     const uint32_t tmem = tmem_s;
+    bool complete = true;                                           // readers: the sums are
 
     if (warp == TC_WARP_TMA) {
         if (elect_one()) {
@@ -149,7 +151,7 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
         }
         __syncwarp();
     } else {
-        tc::wait_uniform(&acc_full, 0, abort_flag);
+        complete = tc::wait_uniform(&acc_full, 0, abort_flag);
         tc::tc_fence_after();
     }
 
@@ -157,7 +159,7 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
     const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16);
     const bool reader = warp < 4 && warp * 32 < rows;
     if (g.splits == 1) {
-        if (reader) {
+        if (reader && complete) {
             const int r = warp * 32 + lane;
             const size_t row_off = (size_t)(row0 + r) * g.ldc;
 #pragma unroll 1
@@ -195,8 +197,8 @@ gemm_tcs_kernel(const __grid_constant__ TcsArgs g)
                     *reinterpret_cast<float4*>(to + c0 + j) = make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
             }
         }
-        cluster_sync_all();
-        for (int i = tid; i < own * (OUT / 4); i += TC_THREADS) {
+        const bool all_ok = cluster_meet(abort_flag);
+        for (int i = tid; i < own * (OUT / 4) && all_ok; i += TC_THREADS) {
             const int r = i / (OUT / 4), col = (i - r * (OUT / 4)) * 4, m = rank * own + r;
             if (m >= rows || n0 + col >= g.N) continue;
             const float4 x = cluster_sum4(sums + m * LD + col, g.splits);

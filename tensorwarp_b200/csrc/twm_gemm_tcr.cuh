@@ -102,6 +102,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     __syncthreads();
     pdl_launch_dependents();
     volatile int* abort_flag = &sm.abort_flag;
+    if (p.splits > 1) cluster_started();
 
     // A whole tile inside N with 16-byte aligned scale rows: the group's 256 scales (512 bytes) ride along with
     // the group's first packed stage; otherwise the unpack threads read them from global memory.
@@ -251,8 +252,8 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         ok = ok && (*abort_flag == 0);
         const int nb = n0 + cpart * RCOLS;
         if (p.splits > 1) {
-            // The slices of a cluster add up, 128 rows at a time (a CTA whose waits ran out shows what it has, so that the
-            // cluster's barriers are met; the error word is set).
+            // the slices of a cluster add up, 128 rows at a time
+            bool all_ok = true;
             float* sums = reinterpret_cast<float*>(&sm.packed[0][0]);
 #pragma unroll 1
             for (int rb = 0; rb < RB; ++rb) {
@@ -268,8 +269,8 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                     for (int j = 0; j < 16; j += 4)
                         *reinterpret_cast<float4*>(to + c0 + j) = make_float4(__uint_as_float(d[j]), __uint_as_float(d[j + 1]), __uint_as_float(d[j + 2]), __uint_as_float(d[j + 3]));
                 }
-                cluster_sync_all();
-                tcw::slice_sum_store<NT>(p, sums, rb * MB, rows, blockIdx.y, n0, tid, UNPACK_WARPS * 32);
+                if (rb == 0) all_ok = cluster_meet(abort_flag); else cluster_sync_all();
+                if (all_ok) tcw::slice_sum_store<NT>(p, sums, rb * MB, rows, blockIdx.y, n0, tid, UNPACK_WARPS * 32);
                 cluster_sync_all();                            // the sums are overwritten, or the CTA leaves
             }
             ok = false;                                        // stored
@@ -334,7 +335,8 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     }
 
     if (p.splits > 1 && warp >= UNPACK_WARPS) {                // the other warps of the barriers above
-        for (int i = 0; i < 2 * RB; ++i) cluster_sync_all();
+        cluster_meet(abort_flag);
+        for (int i = 1; i < 2 * RB; ++i) cluster_sync_all();
     }
 
     // ------------------------------------------------------------ teardown --

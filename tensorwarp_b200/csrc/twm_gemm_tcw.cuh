@@ -133,6 +133,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     __syncthreads();
     pdl_launch_dependents();
     volatile int* abort_flag = &sm.abort_flag;
+    if (p.cluster_reduce) cluster_started();
 
     // A whole tile inside N with 16-byte aligned scale rows: the group's 128 scales (256 bytes) ride along
     // with the packed stage as one bulk copy; a ragged last tile reads them from global memory instead.
@@ -299,13 +300,11 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         const size_t row_off = (size_t)m * p.ldc + nb;
         const bool full = nb + EPI_COLS <= p.N;
         if (p.cluster_reduce) {
-            // (a CTA whose waits ran out shows what it has, so that the cluster's barriers are met; the error word is set)
             float* sums = reinterpret_cast<float*>(&sm.a[0][0]);       // this CTA's MMAs have run: its stages are free
             float* to = sums + (m - row0) * SLICE_LD<NT> + cbase;
 #pragma unroll
             for (int j = 0; j < EPI_COLS; j += 4) *reinterpret_cast<float4*>(to + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-            cluster_sync_all();
-            slice_sum_store<NT>(p, sums, row0, rows, blockIdx.y, n0, tid, EPI_THREADS);
+            if (cluster_meet(abort_flag)) slice_sum_store<NT>(p, sums, row0, rows, blockIdx.y, n0, tid, EPI_THREADS);
             cluster_sync_all();                              // nobody leaves while its sums may still be read
         } else if (ok && row_ok) {
             if (p.splits == 1) {
@@ -414,7 +413,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     }
 
     if (p.cluster_reduce && warp >= WARP_UNPACK0) {          // the other warps of the two barriers above
-        cluster_sync_all();
+        cluster_meet(abort_flag);
         cluster_sync_all();
     }
 

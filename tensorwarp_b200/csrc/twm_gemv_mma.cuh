@@ -192,7 +192,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
     pdl_launch_dependents();
     // Cluster launches: a CTA may store into the leader's shared memory only once the leader has
     // started.  Everybody arrives here, and waits just before the first such store.
-    if (p.cluster_reduce) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (p.cluster_reduce) cluster_started();
     volatile int* abort_flag = &sm.abort_flag;
 
     float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -516,7 +516,6 @@ gemv_kernel(const __grid_constant__ GemmParams p)
         // the same bits whatever order the slices finish in.  Every thread of every CTA
         // reaches the barrier (all loops above are bounded).
         const uint32_t rank = cluster_ctarank();
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // pairs with the arrive at the top: every CTA of the cluster runs
         if (MP > CLUSTER_ROWS) {
             // three to eight rows: each CTA leaves its sums where its weights were and adds up a share of the tile over the
             // cluster, in slice order (four rows, N=4608, K=3584: 10.2 us through the workspace, 6.5 here; N=2048, K=2048: 10.9 and 4.7)
@@ -527,8 +526,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
                 float* to = sums + mA * LD + wcol + g;
                 to[0] = tot[0]; to[LD] = tot[1]; to[8] = tot[2]; to[LD + 8] = tot[3];
             }
-            cluster_sync_all();
-            if (consumer && *abort_flag == 0)
+            if (cluster_meet(abort_flag) && consumer)
                 for (int i = (int)rank * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
                     const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
                     if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));
@@ -536,6 +534,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
             cluster_sync_all();                                          // nobody leaves while its sums may still be read
             return;
         }
+        cluster_wait_started();
         if (consumer && t == 0 && *abort_flag == 0) {
             const uint32_t base = mapa_shared(smem_u32(&sm.red[rank * p.M][0]), 0);
             st_cluster_f32(base + (wcol + g) * 4, tot[0]);
@@ -545,6 +544,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
                 st_cluster_f32(base + (NT + wcol + g + 8) * 4, tot[3]);
             }
         }
+        cluster_share_abort(abort_flag);
         cluster_sync_all();
         if (rank == 0 && tid < p.M * NT && *abort_flag == 0) {
             const int m = tid / NT, col = tid - m * NT;
@@ -707,6 +707,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
     __syncthreads();
     pdl_launch_dependents();
     volatile int* abort_flag = &sm.abort_flag;
+    if (p.cluster_reduce) cluster_started();
 
     float tot[NTL][4];
 #pragma unroll
@@ -850,7 +851,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
     // lane (g, t): C[m = 8 nt + 2t, + 1][n = n0 + wcol + g] and the same rows for column + 8
     if (warp >= CONSUMER_WARPS) {
         __syncwarp();
-        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers below
+        if (p.cluster_reduce) { cluster_meet(abort_flag); cluster_sync_all(); }      // the barriers below
         return;
     }
     const int nA = n0 + wcol + g, nB = nA + 8;
@@ -881,8 +882,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
             float* to = sums + (nt * 8 + 2 * t) * LD + wcol + g;
             to[0] = tot[nt][0]; to[LD] = tot[nt][1]; to[8] = tot[nt][2]; to[LD + 8] = tot[nt][3];
         }
-        cluster_sync_all();
-        if (*abort_flag == 0)
+        if (cluster_meet(abort_flag))
             for (int i = blockIdx.y * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
                 const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
                 if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));

@@ -95,6 +95,7 @@ gemv_kernel(const GemmParams p)
     pdl_launch_dependents();
 
     volatile int* abort_flag = &sm.abort_flag;
+    if (p.cluster_reduce) cluster_started();
 
     if (warp == SB) {
         // ------------------------------------------------------- producer --
@@ -147,7 +148,7 @@ gemv_kernel(const GemmParams p)
             }
             __syncwarp();
         }
-        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers at the end
+        if (p.cluster_reduce) { cluster_meet(abort_flag); cluster_sync_all(); }      // the barriers at the end
         return;
     }
 
@@ -271,7 +272,7 @@ gemv_kernel(const GemmParams p)
 
     // ------------------------------------------- reduce the eight warps --
     named_bar_sync(1, CONSUMERS);
-    if (*abort_flag && !p.cluster_reduce) return;   // a wait expired: leave C untouched, the error word is set
+    if (*abort_flag && !p.cluster_reduce) return;   // a wait expired: leave C untouched, the error word is set (a cluster: at cluster_meet)
     float* red = reinterpret_cast<float*>(&sm.packed[0][0]);   // [SB][MMAX][NT], ring is idle now
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -321,8 +322,7 @@ gemv_kernel(const GemmParams p)
 #pragma unroll
             for (int m = 0; m < MMAX; ++m) sums[m * NT + tid] = part[m];
         }
-        cluster_sync_all();
-        if (*abort_flag == 0)
+        if (cluster_meet(abort_flag))
             for (int i = tid * p.splits + blockIdx.y; i < p.M * (NT / 4); i += CONSUMERS * p.splits) {
                 const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
                 if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * NT + c, p.splits));

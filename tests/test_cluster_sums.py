@@ -1,0 +1,39 @@
+"""CTAs of a cluster that add up one another's sums: no CTA stores C when a wait of any of them ran out.  Read from the sources: a wait
+that runs out leaves copies in flight, so none is made to on a GPU."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tensorwarp_b200", "csrc")
+FILES = {"twm_gemv_simt.cuh": 1, "twm_gemv_mma.cuh": 2, "twm_gemm_tcw.cuh": 1, "twm_gemm_tcr.cuh": 1, "twm_dense_tcs.cuh": 1, "twm_dense_f32tc.cuh": 1}
+
+
+def kernels(name):
+    """Bodies of the kernels of a file that read sums of other CTAs or push sums to them, without comments."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    bodies = [b for b in text.split("__global__")[1:]]
+    return [b for b in bodies if re.search(r"cluster_sum4\(|slice_sum_store<|st_cluster_f32\(", b)]
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_no_cta_of_a_cluster_stores_after_an_expired_wait(name):
+    found = kernels(name)
+    assert len(found) == FILES[name]
+    for body in found:
+        assert body.count("cluster_started();") == 1
+        meet = body.index("cluster_meet(abort_flag)" if "cluster_meet(abort_flag)" in body else "cluster_share_abort(abort_flag)")
+        for use in re.finditer(r"cluster_sum4\(|slice_sum_store<", body):
+            before = body[meet:use.start()]
+            assert meet < use.start()
+            # the statement that stores hangs on what cluster_meet returned
+            assert re.search(r"if \(cluster_meet\(abort_flag\)|if \(all_ok\)|&& all_ok|if \(!all_ok\)", body[max(0, meet - 40):use.start()]), before
+        for push in re.finditer(r"st_cluster_f32\(", body):          # partial sums pushed to a leader, which looks at its own flag
+            tail = body[push.start():]
+            assert tail.index("cluster_share_abort(abort_flag)") < tail.index("cluster_sync_all()") < tail.index("*abort_flag == 0")
+
+
+def test_every_wait_ends_and_every_cta_meets():
+    """The warps that do not add up reach the same barriers: one meeting and the closing barrier."""
+    for name in ("twm_gemv_simt.cuh", "twm_gemm_tcw.cuh", "twm_gemm_tcr.cuh"):
+        assert kernels(name)[0].count("cluster_meet(abort_flag)") == 2
