@@ -407,11 +407,8 @@ twm_status gemm_tcs_launch(const bf16* a, int lda, const bf16* w, int ldw, void*
 template <int EPI>
 twm_status gemm_tcs(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, int M, int N, int K, const TcsPlan& plan, int flags, void* stream)
 {
-    switch (plan.bn) {
-        case 256: return gemm_tcs_launch<256, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
-        case 128: return gemm_tcs_launch<128, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
-        default: return gemm_tcs_launch<64, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
-    }
+    return plan.bn == 128 ? gemm_tcs_launch<128, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream)
+                          : gemm_tcs_launch<64, EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
 }
 
 // Whether the product of few tiles takes a call (bn > 0), and how; tile and stage_cost are tc_tile_choice's.
@@ -488,14 +485,14 @@ twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, i
 {
     int sms = 148;
     TRY(device(&sms));
-    GemmF32Args g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, 1, 1};
+    GemmF32Args g = {a, w, (float*)c, lda, ldw, ldc, M, N, K, 1};
     const int out = EPI == TWM_EPI_GELU_GLU ? F32_BN / 2 : F32_BN, n_tiles = (N + out - 1) / out, k_tiles = (K + F32_BK - 1) / F32_BK;
     long best = -1;
     for (int s = 1; s <= F32_MAX_SPLITS; ++s) {
         const long waves = ((long)n_tiles * s + 2 * sms - 1) / (2 * sms), cost = waves * ((k_tiles + s - 1) / s + (s > 1 ? 8 : 0));
         if (best < 0 || cost < best) { best = cost; g.splits = s; }
     }
-    return launch("gemm_f32", gemm_f32_kernel<1, EPI>, dim3((unsigned)((long)n_tiles * g.splits)), F32_THREADS, f32_smem_bytes(1), flags, stream,
+    return launch("gemm_f32", gemm_f32_kernel<EPI>, dim3((unsigned)((long)n_tiles * g.splits)), F32_THREADS, F32_SMEM_BYTES, flags, stream,
                   g.splits > 1 ? g.splits : 0, g);
 }
 // From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 5 rows 2.37 / 2.72,

@@ -1,7 +1,7 @@
 // twm_dense_f32.cuh — C[M][N] = A[M][K] . W[N][K]^T of the 32-bit models for up to eight rows, in FP32 FMAs.
 //
-// Bound by reading W.  Tile 8 TM rows x 128 weight rows, 32 K a stage, three
-// stages of 16-byte asynchronous copies, two CTAs to an SM.  A thread has TM x 4 sums, each as a PAIR over even and odd K
+// Bound by reading W.  Tile 8 rows x 128 weight rows, 32 K a stage, three stages of 16-byte asynchronous copies, two CTAs to an SM.
+// A thread has one row x 4 weight rows' sums, each as a PAIR over even and odd K
 // (fma.rn.f32x2: two FMAs an instruction), so both operands stay in shared memory as they lie in global memory, rows of K
 // padded by 16 bytes: a quarter warp reads eight consecutive rows without conflicts, and an operand needs no transposition.
 //
@@ -17,32 +17,32 @@
 namespace twm {
 namespace dense {
 
-constexpr int F32_BK = 32, F32_LD = F32_BK + 4, F32_BN = 128, F32_THREADS = 256, F32_STAGES = 3, F32_MAX_SPLITS = 8;
-__host__ __device__ constexpr int f32_stage_floats(int tm) { return (8 * tm + F32_BN) * F32_LD; }
-__host__ __device__ constexpr size_t f32_smem_bytes(int tm) { return sizeof(float) * (size_t)F32_STAGES * f32_stage_floats(tm); }
+constexpr int F32_ROWS = 8, F32_BK = 32, F32_LD = F32_BK + 4, F32_BN = 128, F32_THREADS = 256, F32_STAGES = 3, F32_MAX_SPLITS = 8;
+constexpr int F32_STAGE_FLOATS = (F32_ROWS + F32_BN) * F32_LD;
+constexpr size_t F32_SMEM_BYTES = sizeof(float) * (size_t)F32_STAGES * F32_STAGE_FLOATS;
 
 struct GemmF32Args {
     const float *a, *w;
     float* c;
     int lda, ldw, ldc, M, N, K;     // gated: N output columns, 2 N weight rows
-    int m_tiles, splits;
+    int splits;
 };
 
 __device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-template <int TM, int EPI>
+template <int EPI>
 __global__ void __launch_bounds__(F32_THREADS, 2)
 gemm_f32_kernel(const GemmF32Args g)
 {
     constexpr bool GATED = EPI == TWM_EPI_GELU_GLU;
-    constexpr int BM = 8 * TM, TN = F32_BN / 32, OUT = GATED ? F32_BN / 2 : F32_BN, STAGE = f32_stage_floats(TM);
+    constexpr int BM = F32_ROWS, TN = F32_BN / 32, OUT = GATED ? F32_BN / 2 : F32_BN, STAGE = F32_STAGE_FLOATS;
     extern __shared__ __align__(16) float f32_smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31;
     const int rank = blockIdx.x % g.splits, tile = blockIdx.x / g.splits;
-    const int m0 = tile % g.m_tiles * BM, n0 = tile / g.m_tiles * OUT;
+    const int n0 = tile * OUT;
     const int k_tiles = (g.K + F32_BK - 1) / F32_BK, per = (k_tiles + g.splits - 1) / g.splits;
     const int k_first = min(k_tiles, rank * per), steps = min(k_tiles, k_first + per) - k_first;
 
@@ -62,13 +62,9 @@ gemm_f32_kernel(const GemmF32Args g)
     auto load_a = [&](int step) {
         float* as = f32_smem + (step % F32_STAGES) * STAGE;
         const int k = (k_first + step) * F32_BK + piece, bytes = max(0, min(4, g.K - k)) * 4;
-#pragma unroll
-        for (int i = 0; i < (BM + 31) / 32; ++i) {
-            const int r = row0 + i * 32;
-            if (BM % 32 && r >= BM) break;
-            const bool in = m0 + r < g.M && bytes > 0;
-            ops::att_cp_async16(smem_u32(as + r * F32_LD + piece), g.a + (in ? (size_t)(m0 + r) * g.lda + k : 0), in ? bytes : 0);
-        }
+        if (row0 >= BM) return;
+        const bool in = row0 < g.M && bytes > 0;
+        ops::att_cp_async16(smem_u32(as + row0 * F32_LD + piece), g.a + (in ? (size_t)row0 * g.lda + k : 0), in ? bytes : 0);
     };
     // weights are constants: the first stages of them are on their way before the preceding kernel has ended
 #pragma unroll
@@ -81,12 +77,10 @@ gemm_f32_kernel(const GemmF32Args g)
         ops::att_cp_async_commit();
     }
 
-    const int tr = lane & 7, tc = (tid >> 5) * 4 + (lane >> 3);     // rows tr + 8 i, weight rows tc + 32 j
-    uint64_t acc[TM][TN];
+    const int tr = lane & 7, tc = (tid >> 5) * 4 + (lane >> 3);     // row tr, weight rows tc + 32 j
+    uint64_t acc[TN];
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+    for (int j = 0; j < TN; ++j) acc[j] = 0;
     for (int step = 0; step < steps; ++step) {
         asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
         __syncthreads();                                            // the stage is there, and the one before it has been used
@@ -96,14 +90,12 @@ gemm_f32_kernel(const GemmF32Args g)
         const float* ws = f32_smem + (step % F32_STAGES) * STAGE + (BM + tc) * F32_LD;
 #pragma unroll
         for (int k = 0; k < F32_BK; k += 4) {
-            ulonglong2 wv[TN];
+            const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(as + k);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 32 * F32_LD + k);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(as + i * 8 * F32_LD + k);
-#pragma unroll
-                for (int j = 0; j < TN; ++j) { fma2(acc[i][j], av.x, wv[j].x); fma2(acc[i][j], av.y, wv[j].y); }
+            for (int j = 0; j < TN; ++j) {
+                const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(ws + j * 32 * F32_LD + k);
+                fma2(acc[j], av.x, wv.x);
+                fma2(acc[j], av.y, wv.y);
             }
         }
     }
@@ -111,28 +103,25 @@ gemm_f32_kernel(const GemmF32Args g)
     // every CTA of the cluster has used its stages; the sums go to the owners of their rows
     const int own = (BM + g.splits - 1) / g.splits;
     if (g.splits > 1) cluster_sync_all(); else __syncthreads();
+    const int owner = g.splits > 1 ? tr / own : 0;
+    float* to = f32_smem + ((size_t)rank * own + (tr - owner * own)) * F32_BN + tc;
+    const uint32_t remote = g.splits > 1 ? mapa_shared(smem_u32(to), owner) : 0;
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = tr + 8 * i, owner = g.splits > 1 ? m / own : 0;
-        float* to = f32_smem + ((size_t)rank * own + (m - owner * own)) * F32_BN + tc;
-        const uint32_t remote = g.splits > 1 ? mapa_shared(smem_u32(to), owner) : 0;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const float v = __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
-            if (g.splits > 1) st_cluster_f32(remote + j * 32 * 4, v);
-            else to[j * 32] = v;
-        }
+    for (int j = 0; j < TN; ++j) {
+        const float v = __uint_as_float((uint32_t)acc[j]) + __uint_as_float((uint32_t)(acc[j] >> 32));
+        if (g.splits > 1) st_cluster_f32(remote + j * 32 * 4, v);
+        else to[j * 32] = v;
     }
     if (g.splits > 1) cluster_sync_all(); else __syncthreads();
     for (int i = tid; i < own * OUT; i += F32_THREADS) {
         const int r = i / OUT, n = i - r * OUT, m = rank * own + r;
-        if (m >= BM || m0 + m >= g.M || n0 + n >= g.N) continue;
+        if (m >= g.M || n0 + n >= g.N) continue;
         float v = 0.0f, up = 0.0f;
         for (int s = 0; s < g.splits; ++s) {
             v += f32_smem[((size_t)s * own + r) * F32_BN + n];
             if (GATED) up += f32_smem[((size_t)s * own + r) * F32_BN + OUT + n];
         }
-        g.c[(size_t)(m0 + m) * g.ldc + n0 + n] = GATED ? gelu_tanh(v) * up : epilogue_value<EPI>(v);
+        g.c[(size_t)m * g.ldc + n0 + n] = GATED ? gelu_tanh(v) * up : epilogue_value<EPI>(v);
     }
 }
 
