@@ -168,7 +168,10 @@ typedef struct twm_plan_t {
     int grid_x, grid_y;  /* n tiles, splits */
     size_t workspace_bytes;
     int cluster_reduce;  /* 1: the K slices of a tile run as one thread-block cluster and add up in
-                            distributed shared memory; no workspace is touched */
+                            distributed shared memory; no workspace is asked for.  0 with splits > 1: room for
+                            the slices is asked for, although up to 8 slices of three rows or more on the
+                            streaming MMA kernel, and up to 16 of up to four rows on the FP32 kernel, add up
+                            as a cluster as well and leave it alone */
 } twm_plan_t;
 
 /* Replaces the adaptive split-K arithmetic of quantize.rs:1314-1325, re-derived

@@ -416,9 +416,9 @@ twm_status gemm_tcs(const bf16* a, int lda, const bf16* w, int ldw, void* c, int
 // the exchange of the sums (fitted to 40 products of 4 to 700 rows: the choice is within 4 % of the best on average).  Clusters that
 // would not all run at once cost twice that, so they are not taken: 18 clusters of 8 do not fit 148 SMs.
 // Not shared, one CTA a tile: where the plain product would take one wave of 64- or 128-column tiles, which the even rows and
-// the single accumulator do no slower (2 rows, 8208 x 2048: 16.0 -> 9.1 us; 100 rows: 9.4 -> 9.0); and for up to 128 rows in several
-// waves, two CTAs to an SM so that one loads while the other stores (2 rows, 18944 gated x 3584: 50.7 -> 43.1 us; 100 rows: 47.6 ->
-// 46.4).  From 65 rows on and more than two CTAs an SM the persistent product is faster (128 rows, 152064 x 3584: 210 against 225 us).
+// the single accumulator do no slower (2 rows, 8208 x 2048: 17.9 -> 10.9 us; 100 rows: 10.9 both); and for up to 128 rows in several
+// waves, two CTAs to an SM so that one loads while the other stores (2 rows, 18944 gated x 3584: 52.9 -> 44.1 us; 100 rows: 48.9 ->
+// 47.9).  From 65 rows on and more than two CTAs an SM the persistent product is faster (128 rows, 152064 x 3584: 210 against 225 us).
 twm_status tcs_plan(int M, int N, int K, bool gated, int sms, int tile, long stage_cost, TcsPlan* plan)
 {
     const int m_tiles = (M + TC_BM - 1) / TC_BM, bm = ((M + m_tiles - 1) / m_tiles + 7) / 8 * 8, k_tiles = (K + TC_BK - 1) / TC_BK;
@@ -496,8 +496,8 @@ twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, i
                   g.splits > 1 ? g.splits : 0, g);
 }
 // From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 5 rows 2.37 / 2.72,
-// 9 rows 2.80 / 2.75, 20 rows 3.33 / 2.84, 70 rows 6.45 / 3.51, 256 rows 18.2 / 8.1; error against 64 bits of 70 rows x 2048 x 8192:
-// 4.1e-7 / 1.5e-7.
+// 9 rows 2.80 / 2.78, 20 rows 3.33 / 2.88, 70 rows 6.45 / 3.58, 256 rows 18.2 / 8.2; error against 64 bits of 70 rows x 2048 x 8192:
+// 4.1e-7 / 1.2e-7.
 // Error against 64 bits over the sum of absolute products (largest, RMS), 70 rows, FP32 FMAs / tensor cores: K = 1 6.0e-8, 2.5e-8 / 8.9e-8,
 // 2.6e-8; K = 2 1.1e-7, 2.6e-8 / 1.5e-7, 2.2e-8; K = 8 1.9e-7, 2.7e-8 / 1.3e-7, 1.5e-8; K = 1024 2.4e-7, 2.8e-8 / 2.7e-8, 4.6e-9: sums of
 // fewer than eight products stay on the plain tiles.

@@ -1,6 +1,6 @@
 // twm_dense_simt.cuh — FP32-arithmetic tiles for any size and either element type: the matrix
 // product and the windowed sigmoid attention.  The 32-bit models run their attention on these, and products whose rows are
-// not on 16-byte boundaries; the 16-bit ones where the tensor-core kernels' size rules do not hold.
+// not on 16-byte boundaries or that sum up fewer than eight terms; the 16-bit ones where the tensor-core kernels' size rules do not hold.
 #pragma once
 
 #include "twm_dense_common.cuh"

@@ -7,8 +7,10 @@
 // of a cluster accumulates its share of K in TMEM and leaves the sums in its shared memory, where the stages were; each adds up its
 // share of the rows over the cluster in rank order: the same result every time, no workspace.
 //
-// Weights cold, against twm_dense_tc.cuh: 2048 x 8192, 100 rows: 26.3 -> 11.3 us (K over four), 333 rows: 27.6 -> 18.9; 3584 x 18944,
-// 100 rows: 59.8 -> 29.2 us (4.6 TB/s); 2048 x 2048, 100 rows: 8.6 -> 6.6; 5120 x 2048, 2 rows: 16.7 -> 6.7.  Tiles of 256 columns
+// A chain of calls in a graph, weights cold, against twm_dense_tc.cuh: 2048 x 8192, 100 rows: 27.2 -> 12.1 us (K over four), 333 rows:
+// 27.6 -> 19.7; 3584 x 18944, 100 rows: 58.6 -> 29.1 us (4.7 TB/s); 2048 x 2048, 100 rows: 10.2 -> 8.0; 5120 x 2048, 2 rows: 15.0 -> 8.7;
+// a router's 64 x 2048, 4096 rows: 9.6 -> 7.2, and its error against 64 bits 2.1e-6 -> 4.7e-7 of the results: the tensor core cuts
+// when it adds, and a share of K is a shorter sum.  Tiles of 256 columns
 // gained only at 333 rows x 3584 x 18944 (51 instead of 62 us) and lost elsewhere, half the stages with two CTAs to an SM
 // lost wherever one CTA an SM is enough.
 #pragma once

@@ -20,7 +20,7 @@
 // (thread = activation row, 64 columns).  Warp 16: TMA producer.  Warp 17: MMA issuer.  K order inside an
 // 8-wide core is k0,k4,k1,k5,k2,k6,k3,k7 as in the other tcgen05 kernels (the pre-pass writes the
 // activations that way).  Fewer tiles than SMs: K is cut into slices, a cluster of up to eight CTAs a tile (see twm_gemm_tcw.cuh); 200
-// rows, weights cold: N=4608, K=3584 53.4 us in one slice, 24.7 in six; N=3584: 53.6 and 23.2; N=18944: 54.6 and 36.9 in two.  One CTA per SM (about 180 KB of shared memory), 256 TMEM columns.
+// rows, weights cold: N=4608, K=3584 52.8 us in one slice, 25.2 in six; N=3584: 53.6 and 23.2; N=18944: 54.6 and 36.9 in two.  One CTA per SM (about 180 KB of shared memory), 256 TMEM columns.
 #pragma once
 
 #include "twm_common.cuh"

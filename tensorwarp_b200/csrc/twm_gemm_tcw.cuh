@@ -25,7 +25,7 @@
 // shared memory, all 512 TMEM columns: four accumulators).
 //
 // Where the tiles leave SMs idle, K is cut into slices of whole scale groups (grid y), a cluster of up to eight CTAs a tile, whose
-// sums add up over the cluster's shared memory.  Weights cold, 128 rows: N=3584, K=3584: 29.2 us in one slice, 14.4 in four;
+// sums add up over the cluster's shared memory.  Weights cold, 128 rows: N=3584, K=3584: 29.2 us in one slice, 14.6 in four;
 // K=18944: 122 and 38.9 us (64 in five slices through the workspace, whose partials and last arriver's sum cost 7 us a slice).
 // 200 rows, K=18944: 115 us as two such launches, 69 as one launch of 2 x 28 tiles in two slices.
 #pragma once

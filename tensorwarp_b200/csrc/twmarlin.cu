@@ -288,14 +288,15 @@ int auto_kernel(int M, int N, int K, int G, bool a_is_f16, bool indirect, int sp
 {
     if (!a_is_f16) return TWM_KERNEL_SIMT;
     (void)K;
-    // many rows: rows on the MMA's M dimension; group 128 and full 128-column tiles.  Wide matrices (at least half
-    // a wave of 256-column tiles, no K slices asked for) take the 256-column kernel, whose weights enter the tensor
-    // core rounded to FP16 as in the reference's batched route; the others the exact-weight kernel, which can split K.
+    // many rows: rows on the MMA's M dimension; group 128 and full 128-column tiles.  Wide matrices, and more than 128 rows
+    // (no K slices asked for), take the 256-column kernel, whose weights enter the tensor core rounded to FP16 as in the
+    // reference's batched route; the others the exact-weight kernel.
     if (M >= kTcwFromRows && G == 128 && N >= 128 && !indirect) {
         // Measured on K=3584 (us, 128 / 256 rows, each with the K slices of its plan): N=37888: tcr 46 / 61, tcw 57 / 110; N=18944:
-        // 28 / 39 against 30 / 56; N=4608: 18 / 27 against 17 / 21.  K=18944, N=3584: 37 / 52 against 39 / 70.  So: more than one wave
-        // of 128-column tiles, or more than 128 rows, goes to the 256-column kernel unless K is long and the tiles are few, where
-        // the exact weights stay.
+        // 28 / 39 against 30 / 56; N=4608: 18 / 27 against 17 / 21.  K=18944, N=3584: 37 / 52 against 39 / 70.  More than one wave of
+        // 128-column tiles, or more than 128 rows, goes to the 256-column kernel, which these figures bear out from N=18944 on.  Two
+        // lines are older than the slices: narrow matrices of 129 to 256 rows go there too, where the exact weights would now
+        // be faster (N=4608: 21 against 27), and a long K with few tiles stays with the exact weights, which are slower by now.
         const int tiles_w = (N + twm::tcw::NT - 1) / twm::tcw::NT, tiles_r = (N + twm::tcr::NT - 1) / twm::tcr::NT;
         const bool long_k_few_tiles = K >= 8192 && 4 * tiles_r <= kDefaultSms;
         const bool wide = (tiles_w > kDefaultSms || M > twm::tcw::MB) && !long_k_few_tiles && splits_override <= 1;
