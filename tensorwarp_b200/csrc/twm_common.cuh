@@ -202,6 +202,26 @@ __device__ __forceinline__ bool cluster_meet(volatile int* abort_flag) {
     cluster_sync_all();
     return *abort_flag == 0;
 }
+// The same where a thread reads a sum or two of each CTA: cluster_sum4, and whether no wait of any CTA ran out, from loads issued
+// together, without a second barrier (one FP32 row, 16384 x 2048: 10.6 us with cluster_meet, 10.4 this way and without either).
+__device__ __forceinline__ bool cluster_sum4_met(const float* local, volatile int* abort_flag, int n, float4& v) {
+    const uint32_t at = smem_u32(local), flag = smem_u32(const_cast<int*>(abort_flag));
+    uint32_t gave_up = 0;
+    v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = 0; b < n; b += 8) {
+        float4 t[8];
+        uint32_t f[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (b + i < n) {
+                t[i] = ld_cluster_f32x4(mapa_shared(at, b + i));
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(f[i]) : "r"(mapa_shared(flag, b + i)) : "memory");
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (b + i < n) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; gave_up |= f[i]; }
+    }
+    return gave_up == 0;
+}
 
 // --------------------------------------------- system-scope flags (peers) --
 __device__ __forceinline__ void st_release_sys_u32(unsigned int* p, unsigned int v) {

@@ -192,7 +192,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
     pdl_launch_dependents();
     // Cluster launches: a CTA may store into the leader's shared memory only once the leader has
     // started.  Everybody arrives here, and waits just before the first such store.
-    if (p.cluster_reduce) cluster_started();
+    if (MP <= CLUSTER_ROWS && p.cluster_reduce) cluster_started();
     volatile int* abort_flag = &sm.abort_flag;
 
     float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -526,11 +526,12 @@ gemv_kernel(const __grid_constant__ GemmParams p)
                 float* to = sums + mA * LD + wcol + g;
                 to[0] = tot[0]; to[LD] = tot[1]; to[8] = tot[2]; to[LD + 8] = tot[3];
             }
-            if (cluster_meet(abort_flag) && consumer)
-                for (int i = (int)rank * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
-                    const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
-                    if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));
-                }
+            cluster_sync_all();
+            for (int i = (int)rank * CONSUMERS + tid; consumer && i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
+                const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+                float4 v;
+                if (n0 + c < p.N && cluster_sum4_met(sums + m * LD + c, abort_flag, p.splits, v)) store_c4(p, m, n0 + c, v);
+            }
             cluster_sync_all();                                          // nobody leaves while its sums may still be read
             return;
         }
@@ -707,7 +708,6 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
     __syncthreads();
     pdl_launch_dependents();
     volatile int* abort_flag = &sm.abort_flag;
-    if (p.cluster_reduce) cluster_started();
 
     float tot[NTL][4];
 #pragma unroll
@@ -851,7 +851,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
     // lane (g, t): C[m = 8 nt + 2t, + 1][n = n0 + wcol + g] and the same rows for column + 8
     if (warp >= CONSUMER_WARPS) {
         __syncwarp();
-        if (p.cluster_reduce) { cluster_meet(abort_flag); cluster_sync_all(); }      // the barriers below
+        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers below
         return;
     }
     const int nA = n0 + wcol + g, nB = nA + 8;
@@ -882,11 +882,12 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
             float* to = sums + (nt * 8 + 2 * t) * LD + wcol + g;
             to[0] = tot[nt][0]; to[LD] = tot[nt][1]; to[8] = tot[nt][2]; to[LD + 8] = tot[nt][3];
         }
-        if (cluster_meet(abort_flag))
-            for (int i = blockIdx.y * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
-                const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
-                if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * LD + c, p.splits));
-            }
+        cluster_sync_all();
+        for (int i = blockIdx.y * CONSUMERS + tid; i < p.M * (NT / 4); i += p.splits * CONSUMERS) {
+            const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+            float4 v;
+            if (n0 + c < p.N && cluster_sum4_met(sums + m * LD + c, abort_flag, p.splits, v)) store_c4(p, m, n0 + c, v);
+        }
         cluster_sync_all();                                  // nobody leaves while its sums may still be read
         return;
     }

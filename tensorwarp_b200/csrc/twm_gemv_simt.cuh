@@ -26,7 +26,7 @@
 // they are taken from `v >> 8`.
 //
 // Split-K.  Up to sixteen slices of up to four rows are a cluster, whose CTAs each add up a share of the columns in slice order from one
-// another's shared memory (one row, 3072 x 2048: 6.9 -> 5.1 us).  Others write FP32 partials to the caller's workspace; the CTA that
+// another's shared memory (one row, 3072 x 2048: 6.9 -> 5.0 us).  Others write FP32 partials to the caller's workspace; the CTA that
 // arrives last on the tile's counter adds the slices in slice order (so the
 // result does not depend on arrival order), stores C and puts the counter back
 // to zero.  No memset launch, no atomics on C.
@@ -95,7 +95,6 @@ gemv_kernel(const GemmParams p)
     pdl_launch_dependents();
 
     volatile int* abort_flag = &sm.abort_flag;
-    if (p.cluster_reduce) cluster_started();
 
     if (warp == SB) {
         // ------------------------------------------------------- producer --
@@ -148,7 +147,7 @@ gemv_kernel(const GemmParams p)
             }
             __syncwarp();
         }
-        if (p.cluster_reduce) { cluster_meet(abort_flag); cluster_sync_all(); }      // the barriers at the end
+        if (p.cluster_reduce) { cluster_sync_all(); cluster_sync_all(); }      // the barriers at the end
         return;
     }
 
@@ -272,7 +271,7 @@ gemv_kernel(const GemmParams p)
 
     // ------------------------------------------- reduce the eight warps --
     named_bar_sync(1, CONSUMERS);
-    if (*abort_flag && !p.cluster_reduce) return;   // a wait expired: leave C untouched, the error word is set (a cluster: at cluster_meet)
+    if (*abort_flag && !p.cluster_reduce) return;   // a wait expired: leave C untouched, the error word is set (a cluster: with the sums)
     float* red = reinterpret_cast<float*>(&sm.packed[0][0]);   // [SB][MMAX][NT], ring is idle now
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -322,11 +321,12 @@ gemv_kernel(const GemmParams p)
 #pragma unroll
             for (int m = 0; m < MMAX; ++m) sums[m * NT + tid] = part[m];
         }
-        if (cluster_meet(abort_flag))
-            for (int i = tid * p.splits + blockIdx.y; i < p.M * (NT / 4); i += CONSUMERS * p.splits) {
-                const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
-                if (n0 + c < p.N) store_c4(p, m, n0 + c, cluster_sum4(sums + m * NT + c, p.splits));
-            }
+        cluster_sync_all();
+        for (int i = tid * p.splits + blockIdx.y; i < p.M * (NT / 4); i += CONSUMERS * p.splits) {
+            const int m = i / (NT / 4), c = (i % (NT / 4)) * 4;
+            float4 v;
+            if (n0 + c < p.N && cluster_sum4_met(sums + m * NT + c, abort_flag, p.splits, v)) store_c4(p, m, n0 + c, v);
+        }
         cluster_sync_all();                                  // nobody leaves while its sums may still be read
         return;
     }
