@@ -186,19 +186,17 @@ __device__ __forceinline__ void cluster_sync_all() {
 // flag of all (which have started by then), and what cluster_meet returns, the same in all, is whether none did.
 __device__ __forceinline__ void cluster_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_share_abort(volatile int* abort_flag) {
-    if (__builtin_expect(*abort_flag, 0)) {
-        uint32_t n;
-        asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+__device__ __forceinline__ void cluster_tell_abort(volatile int* abort_flag) {
+    uint32_t n;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
 #pragma unroll 1
-        for (uint32_t r = 0; r < n; ++r)
-            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_shared(smem_u32(const_cast<int*>(abort_flag)), r)), "r"(1) : "memory");
-    }
-    __syncwarp();
+    for (uint32_t r = 0; r < n; ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_shared(smem_u32(const_cast<int*>(abort_flag)), r)), "r"(1) : "memory");
 }
 __device__ __forceinline__ bool cluster_meet(volatile int* abort_flag) {
     cluster_wait_started();
-    cluster_share_abort(abort_flag);
+    if (__builtin_expect(*abort_flag, 0)) cluster_tell_abort(abort_flag);
+    __syncwarp();
     cluster_sync_all();
     return *abort_flag == 0;
 }

@@ -536,7 +536,9 @@ gemv_kernel(const __grid_constant__ GemmParams p)
             return;
         }
         cluster_wait_started();
-        if (consumer && t == 0 && *abort_flag == 0) {
+        if (__builtin_expect(*abort_flag, 0)) {
+            cluster_tell_abort(abort_flag);
+        } else if (consumer && t == 0) {
             const uint32_t base = mapa_shared(smem_u32(&sm.red[rank * p.M][0]), 0);
             st_cluster_f32(base + (wcol + g) * 4, tot[0]);
             st_cluster_f32(base + (wcol + g + 8) * 4, tot[2]);
@@ -545,7 +547,6 @@ gemv_kernel(const __grid_constant__ GemmParams p)
                 st_cluster_f32(base + (NT + wcol + g + 8) * 4, tot[3]);
             }
         }
-        cluster_share_abort(abort_flag);
         cluster_sync_all();
         if (rank == 0 && tid < p.M * NT && *abort_flag == 0) {
             const int m = tid / NT, col = tid - m * NT;

@@ -31,8 +31,9 @@ def test_no_cta_of_a_cluster_stores_after_an_expired_wait(name):
             assert meet < use.start()
             assert re.search(r"if \(cluster_meet\(abort_flag\)\)|if \(all_ok\)|&& all_ok|if \(!all_ok\)", body[max(0, meet - 40):use.start()])
         for push in re.finditer(r"st_cluster_f32\(", body):          # partial sums pushed to a leader, which looks at its own flag
-            tail = body[push.start():]
-            assert tail.index("cluster_share_abort(abort_flag)") < tail.index("cluster_sync_all()") < tail.index("*abort_flag == 0")
+            told, tail = body[:push.start()].rindex("cluster_tell_abort(abort_flag)"), body[push.start():]
+            assert body.index("cluster_started();") < body[:told].rindex("cluster_wait_started();") and "cluster_sync_all()" not in body[told:push.start()]
+            assert tail.index("cluster_sync_all()") < tail.index("*abort_flag == 0")
 
 
 def test_every_warp_reaches_the_barriers_of_its_cluster():
