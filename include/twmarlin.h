@@ -67,7 +67,8 @@ enum {
      * streaming packed/scales while the kernel before it in the stream is still
      * running, and waits for that kernel only before it reads `a`, the
      * workspace or `c`.  Set it when the weights are constants (the decode
-     * loop); leave it clear when the preceding kernel writes packed/scales. */
+     * loop); leave it clear when the preceding kernel writes packed/scales: the launch
+     * then waits for that kernel before it touches any memory. */
     TWM_FLAG_PDL = 1,
     TWM_FLAG_ACCUMULATE = 2, /* c += result instead of c = result (residual add fused in the epilogue) */
     /* With TWM_FLAG_PDL: the caller asserts that the kernel launched before this one on the stream

@@ -141,6 +141,12 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 __device__ __forceinline__ void pdl_wait_prior_grids() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The start of a kernel whose caller did not ask for dependent launches (wait_first): it is launched while the one before still
+// runs, but touches no memory and lets nothing follow until that one has ended.  What is saved is the launch itself.
+__device__ __forceinline__ void pdl_begin(bool wait_first) {
+    if (wait_first) pdl_wait_prior_grids();
+    pdl_launch_dependents();
+}
 
 // ------------------------------------------------- thread-block clusters --
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -289,6 +295,7 @@ struct GemmParams {
     int blocks_per_split;
     int cluster_reduce;          // 1: the K slices of a tile form a thread-block cluster and add up in its leader's shared memory
     int accumulate;
+    int wait_first;              // nothing, not even the weights, may be read before the launch before has ended (pdl_begin)
     int no_wait;                 // the caller vouches that nothing this launch touches depends on the launch before it
     const uint32_t* packed_offsets;
     const uint32_t* scales_offsets;

@@ -563,15 +563,21 @@ gemm_kernel(const __grid_constant__ GemmParams p)
 // f16 [rows][lda], rewritten as [K/8][rows][8] with the eight K of a core in the order
 // k0,k4,k1,k5,k2,k6,k3,k7 (the order in which the unpack lays nibbles into the operand).  The values
 // themselves are not touched, so any FP16 activation, subnormals included, enters the products
-// exactly.  One thread per (K core, row).
+// exactly.  One thread per (K core, row); a warp takes four cores of eight rows, so that it reads 64 bytes of a row and
+// writes 128 in a run (a thread a core, its lanes on 32 rows, reads 16 bytes of each).
+constexpr int PERM_ROWS = 8, PERM_CORES = 4;
+__host__ __device__ inline int permute_items(int rows, int kcores) {           // kcores: a multiple of 4 (K of 32)
+    return (rows + PERM_ROWS - 1) / PERM_ROWS * PERM_ROWS * kcores;
+}
 __global__ void __launch_bounds__(256)
-permute_activations_kernel(__half* __restrict__ out, const __half* __restrict__ a, long lda, int rows, int kcores)
+permute_activations_kernel(__half* __restrict__ out, const __half* __restrict__ a, long lda, int rows, int kcores, bool wait_first)
 {
-    pdl_launch_dependents();
+    pdl_begin(wait_first);
     pdl_wait_prior_grids();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= rows * kcores) return;
-    const int kc = idx / rows, m = idx - kc * rows;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x, lane = idx & 31, tile = idx >> 5;
+    const int mtiles = (rows + PERM_ROWS - 1) / PERM_ROWS, kt = tile / mtiles;
+    const int m = (tile - kt * mtiles) * PERM_ROWS + lane / PERM_CORES, kc = kt * PERM_CORES + lane % PERM_CORES;
+    if (m >= rows || kc >= kcores) return;
     const __half* src = a + (size_t)m * lda + (size_t)kc * 8;
     uint4 x;
     if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
@@ -586,7 +592,7 @@ permute_activations_kernel(__half* __restrict__ out, const __half* __restrict__ 
     o.y = __byte_perm(x.x, x.z, 0x7632);              // k1,k5
     o.z = __byte_perm(x.y, x.w, 0x5410);              // k2,k6
     o.w = __byte_perm(x.y, x.w, 0x7632);              // k3,k7
-    reinterpret_cast<uint4*>(out)[idx] = o;
+    reinterpret_cast<uint4*>(out)[(size_t)kc * rows + m] = o;
 }
 
 }  // namespace tc

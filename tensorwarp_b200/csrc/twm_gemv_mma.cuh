@@ -189,7 +189,7 @@ gemv_kernel(const __grid_constant__ GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
     // Cluster launches: a CTA may store into the leader's shared memory only once the leader has
     // started.  Everybody arrives here, and waits just before the first such store.
     if (MP <= CLUSTER_ROWS && p.cluster_reduce) cluster_started();
@@ -642,9 +642,9 @@ struct RowsSmem {
 template <int GSHIFT, int AKIND>
 __global__ void __launch_bounds__(256)
 stage_rows_kernel(uint8_t* __restrict__ bq, float* __restrict__ asum, const __half* __restrict__ A, long lda, int M, int MP,
-                  int K, int nkb)
+                  int K, int nkb, bool wait_first)
 {
-    pdl_launch_dependents();
+    pdl_begin(wait_first);
     pdl_wait_prior_grids();
     constexpr int gshift = GSHIFT;
     constexpr int gmask = (1 << gshift) - 1;

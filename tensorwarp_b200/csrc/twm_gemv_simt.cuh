@@ -92,7 +92,7 @@ gemv_kernel(const GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
 
     volatile int* abort_flag = &sm.abort_flag;
 
