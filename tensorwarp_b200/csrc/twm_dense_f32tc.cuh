@@ -27,11 +27,12 @@ namespace dense {
 
 constexpr int FX_BN = 128, FX_BK = 64, FX_MAX_ROWS = 128, FX_CORES = FX_BK / 8;
 constexpr int FX_READERS = 256, FX_SPLITTERS = 256, FX_THREADS = FX_READERS + FX_SPLITTERS + 32, FX_LD = FX_BN + 4;
-// an operand part: [K core of 8][row][16 bytes], cores 16 bytes apart so that eight threads on a row write to distinct banks
-__host__ __device__ constexpr int fx_core_bytes(int rows) { return rows * 16 + 16; }
-__host__ __device__ constexpr int fx_part_bytes(int rows) { return FX_CORES * fx_core_bytes(rows); }
+// An operand part: [row][64 K], 128 bytes a row, its 16-byte pieces in the order of the 128-byte swizzle: the eight threads on a row write
+// one line, and the MMA reads whole lines.  (K cores of 8 x 16 bytes, 16 bytes apart so that the writes met no bank twice, lay across
+// the lines: gate/up of a 70-row prompt, 16384 x 2048, 72.4 us against 66.6; out and down 35.9 against 29.8 on average.)
+__host__ __device__ constexpr int fx_part_bytes(int rows) { return rows * FX_BK * 2; }
 __host__ __device__ constexpr int fx_stage_bytes(int bm) { return 3 * (fx_part_bytes(FX_BN) + fx_part_bytes(bm)); }
-inline size_t fx_smem_bytes(int bm) { return std::max(2 * fx_stage_bytes(bm), bm * FX_LD * 4) + 128; }
+inline size_t fx_smem_bytes(int bm) { return std::max(2 * fx_stage_bytes(bm), bm * FX_LD * 4) + 1024; }
 
 constexpr float FX_SCALE = 16777216.0f, FX_UNSCALE = 1.0f / (FX_SCALE * FX_SCALE);     // 2^24 and 2^-48
 
@@ -91,7 +92,8 @@ gemm_f32tc_kernel(const GemmFxArgs g)
 {
     constexpr bool GATED = EPI == TWM_EPI_GELU_GLU;
     constexpr int OUT = GATED ? FX_BN / 2 : FX_BN;
-    extern __shared__ __align__(128) uint8_t fx_smem[];
+    extern __shared__ uint8_t fx_smem_raw[];
+    uint8_t* fx_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fx_smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t full[2], empty[2], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_s;
     __shared__ int abort_s;
@@ -129,7 +131,6 @@ gemm_f32tc_kernel(const GemmFxArgs g)
         // ------------------------------------------------------------ MMAs --
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bm >> 3) << 17) | ((uint32_t)(FX_BN >> 4) << 24);
-            const uint32_t w_core = fx_core_bytes(FX_BN), a_core = fx_core_bytes(g.bm);
             bool ok = true;
             for (int t = 0; t < steps && ok; ++t) {
                 const int s = t & 1;
@@ -139,13 +140,12 @@ gemm_f32tc_kernel(const GemmFxArgs g)
                 const uint32_t base = smem_u32(fx_smem + s * stage_bytes);
                 // (part of W, part of A): the leading parts into accumulator 0, the five next smaller products into 1
                 auto product = [&](int wp, int ap, uint32_t d, bool first) {
-                    uint64_t wd = tc::make_b_desc(base + wp * w_part, w_core, 128), ad = tc::make_b_desc(base + 3 * w_part + ap * a_part, a_core, 128);
-                    const uint64_t w_step = (2 * w_core) >> 4, a_step = (2 * a_core) >> 4;
+                    uint64_t wd = sw128_desc(base + wp * w_part), ad = sw128_desc(base + 3 * w_part + ap * a_part);
 #pragma unroll
-                    for (int h = 0; h < FX_BK / 16; ++h) {
+                    for (int h = 0; h < FX_BK / 16; ++h) {               // 16 K = 32 bytes further along the swizzled rows
                         tcw::mma_ss(d, wd, ad, idesc, first && h == 0 ? 0u : 1u);
-                        wd += w_step;
-                        ad += a_step;
+                        wd += 2;
+                        ad += 2;
                     }
                 };
                 const uint32_t d = tmem + s * 256;
@@ -164,25 +164,36 @@ gemm_f32tc_kernel(const GemmFxArgs g)
         // ------------------------------------------------------- splitting --
         const int st = tid - FX_READERS, row0 = st >> 3, core = st & 7;      // rows row0 + 32 j, eight K each
         float4 x[8][2];                               // 0-3: weight rows, 4-7: activation rows
-        auto load = [&](int j, int t) {
-            const int r = row0 + (j & 3) * 32, k = (k_first + t) * FX_BK + core * 8;
-            const float* p = nullptr;
+        const int k_lane = k_first * FX_BK + core * 8;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j][0] = x[j][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto load = [&](int j, int t) {               // rows that are not there stay zero
+            const float* p;
             if (j < 4) {
-                const int n = n0 + (GATED ? r % OUT : r);
-                if (n < g.N) p = g.w + (size_t)(GATED && r >= OUT ? g.N + n : n) * g.ldw + k;
-            } else if (r < rows) {
-                p = g.a + (size_t)(m0 + r) * g.lda + k;
+                const int n = n0 + row0 + (GATED ? j & 1 : j) * 32;
+                if (n >= g.N) return;
+                p = g.w + (size_t)(GATED && j >= 2 ? g.N + n : n) * g.ldw;
+            } else {
+                const int r = row0 + (j - 4) * 32;
+                if (r >= rows) return;
+                p = g.a + (size_t)(m0 + r) * g.lda;
+            }
+            p += k_lane + t * FX_BK;
+            const int left = g.K - k_lane - t * FX_BK;
+            if (left >= 8) {
+                x[j][0] = *reinterpret_cast<const float4*>(p);
+                x[j][1] = *reinterpret_cast<const float4*>(p + 4);
+                return;
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 x[j][h] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (p == nullptr) continue;
-                if (k + 4 * h + 4 <= g.K) {
+                if (4 * h + 4 <= left) {
                     x[j][h] = *reinterpret_cast<const float4*>(p + 4 * h);
                 } else {
-                    if (k + 4 * h < g.K) x[j][h].x = p[4 * h];
-                    if (k + 4 * h + 1 < g.K) x[j][h].y = p[4 * h + 1];
-                    if (k + 4 * h + 2 < g.K) x[j][h].z = p[4 * h + 2];
+                    if (4 * h < left) x[j][h].x = p[4 * h];
+                    if (4 * h + 1 < left) x[j][h].y = p[4 * h + 1];
+                    if (4 * h + 2 < left) x[j][h].z = p[4 * h + 2];
                 }
             }
         };
@@ -217,8 +228,9 @@ gemm_f32tc_kernel(const GemmFxArgs g)
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int r = row0 + (j & 3) * 32;
-                if (j < 4) split(j, base + core * fx_core_bytes(FX_BN) + r * 16, w_part);
-                else if (r < g.bm) split(j, base + 3 * w_part + core * fx_core_bytes(g.bm) + r * 16, a_part);
+                uint8_t* piece = base + r * 128 + ((core ^ (r & 7)) << 4);
+                if (j < 4) split(j, piece, w_part);
+                else if (r < g.bm) split(j, piece + 3 * w_part, a_part);
                 if (t + 1 < steps) load(j, t + 1);
             }
             // written through the generic proxy, read by the tensor core through the async proxy
