@@ -316,24 +316,24 @@ twm_status grouped_gemm_tc_launch(const bf16* a, int lda, const bf16* w, int ldw
                   TcCfg<BN>::SMEM_BYTES, flags, stream, 0, g);
 }
 
-template <int EPI>
+template <int BN, int EPI>
 twm_status gemm_tc2_launch(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, int M, int N, int K, int sms, int flags,
                            void* stream)
 {
     constexpr bool gated = EPI == TWM_EPI_GELU_GLU;
-    constexpr int out = gated ? T2_BN / 2 : T2_BN;
+    constexpr int out = gated ? BN / 2 : BN;
     TcArgs g;
     g.c = c; g.ldc = ldc; g.M = M; g.N = N; g.K = K;
     g.m_tiles = (M + 2 * TC_BM - 1) / (2 * TC_BM);
     g.n_tiles = (N + out - 1) / out;
-    if (!rows_map(&g.a_map, a, M, K, lda, TC_BM) || !rows_map(&g.w_map, w, gated ? 2L * N : N, K, ldw, TC_BM))
+    if (!rows_map(&g.a_map, a, M, K, lda, TC_BM) || !rows_map(&g.w_map, w, gated ? 2L * N : N, K, ldw, BN / 2))
         return invalid("cuTensorMapEncodeTiled refused a map of the paired tcgen05 product");
-    return launch("gemm_tc2", gemm_tc2_kernel<EPI>, dim3(2 * std::min(sms / 2, g.m_tiles * g.n_tiles)), TC_THREADS, T2_SMEM_BYTES, flags,
-                  stream, 2, g);
+    return launch("gemm_tc2", gemm_tc2_kernel<BN, EPI>, dim3(2 * std::min(sms / 2, g.m_tiles * g.n_tiles)), TC_THREADS, Tc2Cfg<BN>::SMEM_BYTES,
+                  flags, stream, 2, g);
 }
 
 // Tile: the one whose waves cost least.  Measured time of one 64-K stage of a wave: 0.42, 0.25 and 0.20 us for tiles of
-// 128 rows x 256, 128 and 64 columns; 0.33 us for 256 x 256 on a pair of SMs (returned as 512).
+// 128 rows x 256, 128 and 64 columns; 0.33, 0.29 and 0.255 us for 256 x 256, 224 and 192 on a pair of SMs (returned as 512, 448 and 384).
 int tc_tile_choice(int M, int N, bool gated, int sms, long* stage_cost)
 {
     int best = 256;
@@ -344,11 +344,13 @@ int tc_tile_choice(int M, int N, bool gated, int sms, long* stage_cost)
         const long c = ((tiles + units - 1) / units) * cost;
         if (best_cost < 0 || c < best_cost) { best = choice; best_cost = c; }
     };
-    consider(512, 256, 256, sms / 2, 33);
-    consider(256, 128, 256, sms, 42);
-    consider(128, 128, 128, sms, 25);
-    consider(64, 128, 64, sms, 20);
-    *stage_cost = best_cost;
+    consider(512, 256, 256, sms / 2, 330);
+    consider(448, 256, 224, sms / 2, 290);
+    consider(384, 256, 192, sms / 2, 255);
+    consider(256, 128, 256, sms, 420);
+    consider(128, 128, 128, sms, 250);
+    consider(64, 128, 64, sms, 200);
+    *stage_cost = best_cost / 10;
     return best;
 }
 
@@ -457,7 +459,9 @@ twm_status gemm_tc(const bf16* a, int lda, const bf16* w, int ldw, void* c, int 
         if (plan.bn > 0) return gemm_tcs<EPI>(a, lda, w, ldw, c, ldc, M, N, K, plan, flags, stream);
     }
     switch (width) {
-        case 512: return gemm_tc2_launch<EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
+        case 512: return gemm_tc2_launch<256, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
+        case 448: return gemm_tc2_launch<224, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
+        case 384: return gemm_tc2_launch<192, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
         case 256: return gemm_tc_launch<256, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
         case 128: return gemm_tc_launch<128, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
         default: return gemm_tc_launch<64, EPI>(a, lda, w, ldw, c, ldc, M, N, K, sms, flags, stream);
