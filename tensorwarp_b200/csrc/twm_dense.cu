@@ -837,6 +837,8 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
     // them, and never in chains of sigmoid attention and gated feed-forwards alone); the cause is not known.
     for (int i = 0; i < m->n_layers; ++i)
         if (m->layers[i].mixer != TWM_MIX_SIGMOID || m->layers[i].experts > 0) flags &= ~TWM_FLAG_PDL;
+    int sms = 148;
+    TRY(device(&sms));
     const int wp = m->width_pad;
     float *x = b->x0, *x_next = b->x1;
     const float* y = nullptr;                            // the sublayer output that has yet to join the residual stream
@@ -855,9 +857,10 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
     // the residual stream brought up to date, with the next sublayer's input beside it
     struct Next { const float *shift, *shift_state, *pre_norm, *step; int* clear; int n_clear; };
     auto join = [&](const Next& next, bool want_a) {
-        // rows per CTA: enough CTAs to fill the machine several times; a shifted run computes one row more than it has
-        const int rpc = next.shift ? (rows >= 4096 ? 8 : rows >= 1024 ? 4 : rows >= 256 ? 2 : 1) : 1;
-        const int per = (wp / 4 + ROW_THREADS - 1) / ROW_THREADS;
+        // rows per CTA: those CTAs that run at once (three to an SM for rows of up to 2048 columns, else two) take all; a shifted run computes one
+        // row more than it has
+        const int per = (wp / 4 + ROW_THREADS - 1) / ROW_THREADS, at_once = sms * (per <= 2 ? 3 : 2);
+        const int rpc = per <= 4 ? (rows + at_once - 1) / at_once : next.shift ? (rows >= 4096 ? 8 : rows >= 1024 ? 4 : rows >= 256 ? 2 : 1) : 1;
         const bool full = next.pre_norm || next.step || next.n_clear || routed.rows;
         auto pick = [&](auto f) {
             constexpr bool F = decltype(f)::value;

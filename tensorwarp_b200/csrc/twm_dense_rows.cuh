@@ -118,10 +118,15 @@ __device__ __forceinline__ float4 scale4(const float4 x, float s, const float4 g
 // x_out = residual row; a = T(x_out), or T(token shift of x_out), or T(rms_norm(x_out) * pre_norm).  clear: words set to
 // zero on the way (the expert counts of the routing that follows).  A CTA walks `rows_per_cta` consecutive rows and
 // keeps the row before; its first row's predecessor is computed again (or comes from the state).  PER > 0: a
-// thread's share of a row is PER vectors, held in registers, every load issued before the first use; PER = 0: rows
+// thread's share of a row is PER vectors, held in registers; PER = 0: rows
 // of any length, in shared memory.  FULL = false: without pre_norm, step, routed outputs and clear.
+//
+// Bound by latency: a row is loads, a sum over the CTA, stores.  So the factors are requested before the kernel ahead has ended, and a
+// row's loads before the row ahead of it is worked on (routed: its slots; the experts' rows are all requested at once); the host deals the rows to
+// as many CTAs as run at once.  In a prompt step, a row to a CTA (two rows' work for a shifted one) / this way: 100 rows of 2048 4.6 / 3.9 us,
+// 2048 rows of 3584 35.8 / 28.
 template <typename T, int PER, bool FULL>
-__global__ void __launch_bounds__(ROW_THREADS)
+__global__ void __launch_bounds__(ROW_THREADS, PER == 0 || PER > 4 ? 1 : PER > 2 ? 2 : 3)
 residual_rows_kernel(ResidualSource<T> src, float* __restrict__ x_out, T* __restrict__ a, const float* __restrict__ shift,
                      const float* __restrict__ shift_state, const float* __restrict__ pre_norm, const int* __restrict__ meta, int rows,
                      int rows_per_cta, int* __restrict__ clear, int n_clear)
@@ -129,50 +134,74 @@ residual_rows_kernel(ResidualSource<T> src, float* __restrict__ x_out, T* __rest
     pdl_launch_dependents();
     extern __shared__ __align__(16) float row_smem[];       // PER = 0: [wp], the residual row before
     __shared__ float red[32];
-    pdl_wait_prior_grids();
     const int wp = src.wp, nvec = wp >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+    constexpr bool AHEAD = PER > 0 && PER <= 4;             // the factors are held in registers
+    float4 norms[AHEAD ? PER : 1], factors[AHEAD ? PER : 1];
+    const float* factor_row = shift != nullptr ? shift : FULL ? pre_norm : nullptr;
+    auto norm_at = [&](int i) { return src.y_norm != nullptr ? __ldg(reinterpret_cast<const float4*>(src.y_norm) + i) : one; };
+    auto factor_at = [&](int i) { return factor_row != nullptr ? __ldg(reinterpret_cast<const float4*>(factor_row) + i) : one; };
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int i = threadIdx.x + j * ROW_THREADS;
+            norms[j] = i < nvec ? norm_at(i) : one;
+            factors[j] = i < nvec ? factor_at(i) : one;
+        }
+    }
+    pdl_wait_prior_grids();
     const int r0 = blockIdx.x * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
     const int pos0 = meta[0];
     if (FULL && blockIdx.x == 0)
         for (int i = threadIdx.x; i < n_clear; i += ROW_THREADS) clear[i] = 0;
     const float* st = shift != nullptr && r0 == 0 && pos0 > 0
                           ? shift_state + ((size_t)meta[1] * 2 + ((pos0 - 1) & 1)) * wp : nullptr;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (PER > 0) {
-        __shared__ int slot_row[FULL ? MAX_TOP : 1];
-        __shared__ float slot_weight[FULL ? MAX_TOP : 1];
-        float4 before[PER];
+        __shared__ int slot_row[FULL ? 2 * MAX_TOP : 1];
+        __shared__ float slot_weight[FULL ? 2 * MAX_TOP : 1];
+        const bool is_routed = FULL && src.routed.rows != nullptr;
+        float4 before[PER], x_next[PER], y_next[PER];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             const int i = threadIdx.x + j * ROW_THREADS;
             before[j] = st != nullptr && i < nvec ? reinterpret_cast<const float4*>(st)[i] : zero;
         }
-        for (int r = (shift != nullptr && r0 > 0) ? r0 - 1 : r0; r < r1; ++r) {
-            float4 x[PER], y[PER];
-            if (FULL && src.routed.rows != nullptr) {       // the row's slots, known before the first of their loads
-                __syncthreads();
-                if (threadIdx.x < src.routed.top) {
-                    slot_row[threadIdx.x] = src.routed.row[(size_t)r * src.routed.top + threadIdx.x];
-                    slot_weight[threadIdx.x] = src.routed.weight[(size_t)r * src.routed.top + threadIdx.x];
-                }
-                __syncthreads();
-            }
+        ResidualSource<T> plain = src;                      // the row without what joins it
+        plain.y = nullptr;
+        plain.routed.rows = nullptr;
+        if (!FULL) plain.step = nullptr;
+        auto request = [&](int r) {
             const int tok = src.tokens != nullptr ? src.tokens[r] : 0;
-            ResidualSource<T> plain = src;                  // the row without what joins it
-            plain.y = nullptr;
-            plain.routed.rows = nullptr;
-            if (!FULL) plain.step = nullptr;
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
                 const int i = threadIdx.x + j * ROW_THREADS;
-                y[j] = src.y != nullptr && i < nvec ? src.y_at(r, i) : zero;
-                x[j] = i < nvec ? plain.at(r, pos0 + r, tok, i, 1.0f) : zero;
+                y_next[j] = src.y != nullptr && i < nvec ? src.y_at(r, i) : zero;
+                x_next[j] = i < nvec ? plain.at(r, pos0 + r, tok, i, 1.0f) : zero;
             }
-            if (FULL && src.routed.rows != nullptr) {
-#pragma unroll 4
+        };
+        auto slots_of = [&](int r, int buf) {
+            if (threadIdx.x < src.routed.top) {
+                slot_row[buf * MAX_TOP + threadIdx.x] = src.routed.row[(size_t)r * src.routed.top + threadIdx.x];
+                slot_weight[buf * MAX_TOP + threadIdx.x] = src.routed.weight[(size_t)r * src.routed.top + threadIdx.x];
+            }
+        };
+        const int first = (shift != nullptr && r0 > 0) ? r0 - 1 : r0;
+        if (is_routed) {
+            slots_of(first, 0);
+            __syncthreads();
+        }
+        if (AHEAD) request(first);
+        for (int r = first, buf = 0; r < r1; ++r, buf ^= FULL ? 1 : 0) {
+            float4 x[PER], y[PER];
+            if (!AHEAD) request(r);
+#pragma unroll
+            for (int j = 0; j < PER; ++j) { x[j] = x_next[j]; y[j] = y_next[j]; }
+            if (AHEAD && r + 1 < r1) request(r + 1);
+            if (is_routed) {
+#pragma unroll (PER <= 2 ? 8 : 4)
                 for (int s = 0; s < src.routed.top; ++s) {
-                    const T* row = src.routed.rows + (size_t)slot_row[s] * wp;
-                    const float ws = slot_weight[s];
+                    const T* row = src.routed.rows + (size_t)slot_row[buf * MAX_TOP + s] * wp;
+                    const float ws = slot_weight[buf * MAX_TOP + s];
 #pragma unroll
                     for (int j = 0; j < PER; ++j) {
                         const int i = threadIdx.x + j * ROW_THREADS;
@@ -181,9 +210,10 @@ residual_rows_kernel(ResidualSource<T> src, float* __restrict__ x_out, T* __rest
                         y[j].x = fmaf(t.x, ws, y[j].x); y[j].y = fmaf(t.y, ws, y[j].y); y[j].z = fmaf(t.z, ws, y[j].z); y[j].w = fmaf(t.w, ws, y[j].w);
                     }
                 }
+                if (r + 1 < r1) slots_of(r + 1, buf ^ 1);
             }
             float ir = 1.0f;
-            if ((src.y != nullptr || (FULL && src.routed.rows != nullptr)) && src.y_norm != nullptr) {
+            if ((src.y != nullptr || is_routed) && src.y_norm != nullptr) {
                 float ss = 0.0f;
 #pragma unroll
                 for (int j = 0; j < PER; ++j) ss += ops::sumsq4(y[j]);
@@ -194,8 +224,7 @@ residual_rows_kernel(ResidualSource<T> src, float* __restrict__ x_out, T* __rest
             for (int j = 0; j < PER; ++j) {
                 const int i = threadIdx.x + j * ROW_THREADS;
                 if (i >= nvec) continue;
-                float4 n = make_float4(1.f, 1.f, 1.f, 1.f);
-                if (src.y_norm != nullptr) n = __ldg(reinterpret_cast<const float4*>(src.y_norm) + i);
+                const float4 n = AHEAD ? norms[AHEAD ? j : 0] : norm_at(i);
                 x[j].x += y[j].x * ir * n.x; x[j].y += y[j].y * ir * n.y; x[j].z += y[j].z * ir * n.z; x[j].w += y[j].w * ir * n.w;
                 if (FULL) xs += ops::sumsq4(x[j]);
             }
@@ -207,12 +236,14 @@ residual_rows_kernel(ResidualSource<T> src, float* __restrict__ x_out, T* __rest
                 if (r >= r0) {
                     reinterpret_cast<float4*>(x_out + (size_t)r * wp)[i] = x[j];
                     float4 h = x[j];
-                    if (shift != nullptr) h = shift4(x[j], before[j], __ldg(reinterpret_cast<const float4*>(shift) + i));
-                    if (FULL && pre_norm != nullptr) h = scale4(x[j], pr, __ldg(reinterpret_cast<const float4*>(pre_norm) + i));
+                    const float4 c = AHEAD ? factors[AHEAD ? j : 0] : factor_at(i);
+                    if (shift != nullptr) h = shift4(x[j], before[j], c);
+                    else if (FULL && pre_norm != nullptr) h = scale4(x[j], pr, c);
                     if (a != nullptr) store4<T>(a + (size_t)r * wp + i * 4, h);
                 }
                 before[j] = x[j];
             }
+            if (is_routed) __syncthreads();                 // the next row's slots are there, this one's have been used
         }
     } else {
         if (shift != nullptr) {
@@ -291,9 +322,17 @@ qk_norm_append_kernel(T* __restrict__ proj, int ld, const float* __restrict__ q_
                       const int* __restrict__ meta)
 {
     pdl_launch_dependents();
-    __shared__ float red[32];
-    pdl_wait_prior_grids();
+    __shared__ float red[64];
     using V = Vec<T>;
+    // the factors of a thread's first pieces: on their way before the kernel ahead has ended
+    float4 q_first[V::N / 4], k_first[V::N / 4];
+#pragma unroll
+    for (int j = 0; j < V::N / 4; ++j) {
+        const int i = threadIdx.x * V::N + 4 * j;
+        q_first[j] = q_norm != nullptr && i < q_n ? __ldg(reinterpret_cast<const float4*>(q_norm + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        k_first[j] = k_norm != nullptr && i < k_n ? __ldg(reinterpret_cast<const float4*>(k_norm + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    pdl_wait_prior_grids();
     const int r = blockIdx.x, p = meta[0] + r, slot = meta[1];
     T* row = proj + (size_t)r * ld;
     const bool cached = p < capacity;
@@ -306,12 +345,12 @@ qk_norm_append_kernel(T* __restrict__ proj, int ld, const float* __restrict__ q_
         for (int j = 0; j < V::N; ++j) ss = fmaf(f[j], f[j], ss);
         return ss;
     };
-    auto scaled = [&](const uint4& raw, float ir, const float* g, int i) {
+    auto scaled = [&](const uint4& raw, float ir, const float* g, int i, const float4* ahead) {
         float f[V::N];
         V::unpack(raw, f);
 #pragma unroll
         for (int j = 0; j < V::N; j += 4) {
-            const float4 n = __ldg(reinterpret_cast<const float4*>(g + i * V::N + j));
+            const float4 n = ahead != nullptr ? ahead[j / 4] : __ldg(reinterpret_cast<const float4*>(g + i * V::N + j));
             f[j] *= ir * n.x; f[j + 1] *= ir * n.y; f[j + 2] *= ir * n.z; f[j + 3] *= ir * n.w;
         }
         return V::pack(f);
@@ -339,30 +378,32 @@ qk_norm_append_kernel(T* __restrict__ proj, int ld, const float* __restrict__ q_
 #pragma unroll
         for (int j = 0; j < QP; ++j) qs += sum_sq(q[j]);
         for (int i = threadIdx.x + QP * ROW_THREADS; i < q_n / V::N; i += ROW_THREADS) qs += sum_sq(q_row[i]);
-        const float ir = inv_rms(group_sum(qs, red, ROW_THREADS, 1), q_true, eps);
-#pragma unroll
-        for (int j = 0; j < QP; ++j) {
-            const int i = threadIdx.x + j * ROW_THREADS;
-            if (i < q_n / V::N) reinterpret_cast<uint4*>(row)[i] = scaled(q[j], ir, q_norm, i);
-        }
-        for (int i = threadIdx.x + QP * ROW_THREADS; i < q_n / V::N; i += ROW_THREADS)
-            reinterpret_cast<uint4*>(row)[i] = scaled(q_row[i], ir, q_norm, i);
     }
-    float kir = 1.0f;
     if (k_norm != nullptr) {
 #pragma unroll
         for (int j = 0; j < KP; ++j) ks += sum_sq(k[j]);
         for (int i = threadIdx.x + KP * ROW_THREADS; i < k_n / V::N; i += ROW_THREADS) ks += sum_sq(k_row[i]);
-        kir = inv_rms(group_sum(ks, red, ROW_THREADS, 1), k_true, eps);
+    }
+    const float2 ss = q_norm != nullptr || k_norm != nullptr ? group_sum2(qs, ks, red, ROW_THREADS, 1) : make_float2(0.0f, 0.0f);
+    if (q_norm != nullptr) {
+        const float ir = inv_rms(ss.x, q_true, eps);
+#pragma unroll
+        for (int j = 0; j < QP; ++j) {
+            const int i = threadIdx.x + j * ROW_THREADS;
+            if (i < q_n / V::N) reinterpret_cast<uint4*>(row)[i] = scaled(q[j], ir, q_norm, i, j == 0 ? q_first : nullptr);
+        }
+        for (int i = threadIdx.x + QP * ROW_THREADS; i < q_n / V::N; i += ROW_THREADS)
+            reinterpret_cast<uint4*>(row)[i] = scaled(q_row[i], ir, q_norm, i, nullptr);
     }
     if (cached) {
+        const float kir = k_norm != nullptr ? inv_rms(ss.y, k_true, eps) : 1.0f;
 #pragma unroll
         for (int j = 0; j < KP; ++j) {
             const int i = threadIdx.x + j * ROW_THREADS;
-            if (i < k_n / V::N) reinterpret_cast<uint4*>(k_dst)[i] = k_norm != nullptr ? scaled(k[j], kir, k_norm, i) : k[j];
+            if (i < k_n / V::N) reinterpret_cast<uint4*>(k_dst)[i] = k_norm != nullptr ? scaled(k[j], kir, k_norm, i, j == 0 ? k_first : nullptr) : k[j];
         }
         for (int i = threadIdx.x + KP * ROW_THREADS; i < k_n / V::N; i += ROW_THREADS)
-            reinterpret_cast<uint4*>(k_dst)[i] = k_norm != nullptr ? scaled(k_row[i], kir, k_norm, i) : k_row[i];
+            reinterpret_cast<uint4*>(k_dst)[i] = k_norm != nullptr ? scaled(k_row[i], kir, k_norm, i, nullptr) : k_row[i];
     }
     if (shift_state != nullptr && r == gridDim.x - 1) {
         float* st = shift_state + ((size_t)slot * 2 + (p & 1)) * wp;

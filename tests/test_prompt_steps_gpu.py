@@ -1,13 +1,54 @@
-"""GPU tests of prompt steps at the sizes where their kernels share the work out differently: tiles of 224 and 192 columns on a pair of SMs."""
+"""GPU tests of prompt steps at the sizes where their kernels share the work out differently: rows of several tokens to a CTA, tiles of 224 and
+192 columns on a pair of SMs."""
 import math
 
 import pytest
 import torch
 
-from tensorwarp_b200 import _dense
+import bidasun_cases
+import zukotar_cases
+from tensorwarp_b200 import _dense, dense
+from tensorwarp_b200.engine import DenseEngine
+from tensorwarp_b200.models import bidasun
 from test_dense_ops_gpu import gelu_tanh, gemm
 
 pytestmark = pytest.mark.gpu
+TOL = {torch.float32: 2e-5, torch.bfloat16: 5e-2}
+BOTH = pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+
+
+def bidasun_engine(cfg, dtype, **options):
+    spec, t = bidasun.parse_config(cfg), bidasun_cases.weights(cfg, 7)
+    return DenseEngine(dense.DenseModel(spec, bidasun.model_tensors(spec, lambda n, s: t[n]), dtype), **options)
+
+
+def zukotar_engine(cfg, rank, dtype, **options):
+    return DenseEngine(zukotar_cases.model(cfg, zukotar_cases.weights(cfg, 7, rank), rank, dtype), **options)
+
+
+@BOTH
+@pytest.mark.parametrize("width", [160, 1040, 2064])
+@pytest.mark.parametrize("design", ["bidasun", "zukotar"])
+def test_rows_of_several_tokens_to_a_cta(design, width, dtype):
+    """A prompt whose rows are dealt several to a CTA against the same prompt in portions that are not.  Widths: one, two and three vectors
+    of a row to a thread."""
+    n = 1100 if width < 2000 else 700
+    if design == "bidasun":
+        cfg = bidasun_cases.config(width, 99, [bidasun_cases.layer(bidasun_cases.attention(2, 1, 64, 64, 70, 3), 64),
+                                               bidasun_cases.layer(bidasun_cases.attention(2, 2, 32, 48), 96)], max_positions=1200)
+        make = lambda **o: bidasun_engine(cfg, dtype, **o)
+    else:
+        cfg = zukotar_cases.config(width, 99, [zukotar_cases.layer(zukotar_cases.latent(2, 32, 16, 32, 32, 70), zukotar_cases.experts(2, 2, 32)),
+                                               zukotar_cases.layer(zukotar_cases.linear(2, 32, 32), zukotar_cases.experts(3, 3, 48))])
+        make = lambda **o: zukotar_engine(cfg, 16, dtype, max_tokens=1200, **o)
+    toks, want = bidasun_cases.tokens(cfg, n, 1), sorted({*range(0, n, 7), n - 1})
+    whole = make()
+    got = whole.step(whole.open(), toks, want).clone()
+    parts = make(portion=128)
+    expected = parts.step(parts.open(), toks, want)
+    err = bidasun_cases.error(got.cpu().numpy(), expected.cpu().numpy())
+    assert err.max() < TOL[dtype], (int(err.argmax()), float(err.max()))
+    assert _dense.device_error() == 0
 
 
 @pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
