@@ -630,10 +630,11 @@ twm_status route(const float* logits, const RouterArgs& r, int rows, int* ids, f
 }
 
 template <typename T>
-AttnArgs<T> attn_args(const twm_dense_model* m, const twm_dense_layer& l, const twm_dense_buffers* b, int rows)
+AttnArgs<T> attn_args(const twm_dense_model* m, const twm_dense_layer& l, const twm_dense_buffers* b, int rows, int first_pos)
 {
     const Sizes s = sizes_of(l);
     AttnArgs<T> g;
+    g.first_pos = first_pos;
     g.proj = (const T*)b->proj;
     g.out = (T*)b->att;
     g.k_cache = (const T*)l.k_cache;
@@ -681,7 +682,7 @@ twm_status attention_tc(const AttnArgs<bf16>& g, int end, int slots, int flags, 
     if (!tensor_map(&t.q_map, MapKey{MAP_BF16_SWIZZLED, g.proj, 3, {g.dim_pad, g.heads, g.rows, 0}, {1, g.dim_pad, g.ld, 0}, {64, 1, AT_Q, 0}}) ||
         !cache_map(&t.k_map, g.k_cache, g.dim_pad) || !cache_map(&t.v_map, g.v_cache, g.vdim_pad))
         return invalid("cuTensorMapEncodeTiled refused a map of the tcgen05 attention");
-    return launch("attn_tc", attn_tc_kernel, dim3((g.rows + AT_Q - 1) / AT_Q, g.heads), AT_THREADS, sizeof(AttnTcSmem) + 1024, flags,
+    return launch("attn_tc", attn_tc_kernel, dim3(g.heads, (g.rows + AT_Q - 1) / AT_Q), AT_THREADS, sizeof(AttnTcSmem) + 1024, flags,
                   stream, 0, t);
 }
 twm_status attention_tc(const AttnArgs<float>&, int, int, int, void*) { return invalid("the tcgen05 attention takes bfloat16"); }
@@ -690,7 +691,7 @@ template <typename T>
 twm_status attention(const twm_dense_model* m, const twm_dense_layer& l, const twm_dense_buffers* b, int rows, int first_pos,
                      int kernel, int flags, void* stream)
 {
-    const AttnArgs<T> g = attn_args<T>(m, l, b, rows);
+    const AttnArgs<T> g = attn_args<T>(m, l, b, rows, first_pos);
     if (kernel < 0 || kernel > 3) return invalid("kernel");
     if (kernel == 3 && !attention_tc_fits(g)) return invalid("the tcgen05 attention takes bfloat16 heads of up to 128 columns");
     if (kernel == 3 || (kernel == 0 && attention_tc_fits(g))) return attention_tc(g, first_pos + rows, m->slots, flags, stream);

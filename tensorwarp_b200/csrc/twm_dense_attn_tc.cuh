@@ -1,7 +1,8 @@
 // twm_dense_attn_tc.cuh — windowed sigmoid attention of a portion of a prompt on the 5th-generation tensor
 // cores, bfloat16, heads of up to 128 columns.
 //
-// CTA = 128 queries of one head.  It walks the 128-key tiles that hold a visible key: those of the kept
+// CTA = 128 queries of one head; those with the most keys start first, so that the last wave is made of short ones (2048 queries, 28
+// heads, window 1024: 14 layers of a prompt 13.57 -> 13.32 ms).  It walks the 128-key tiles that hold a visible key: those of the kept
 // first keys, then the window's.  Since the weights are not normalised over keys there is no running
 // maximum and nothing is ever rescaled: S = Q K^T goes to tensor memory, eight warps turn it into weights,
 // and O += P V accumulates in tensor memory over all tiles.
@@ -88,10 +89,11 @@ attn_tc_kernel(const __grid_constant__ AttnTcArgs args)
     tc::tc_fence_after();
     volatile int* abort_flag = &sm.abort_flag;
     const uint32_t tmem = sm.tmem_base, tmem_o = tmem + AT_K;
+    const int h = blockIdx.x, kvh = h / (g.heads / g.kv_heads);
+    const int r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * AT_Q;         // the queries that see most keys first
+    g.prefetch_bias(h, r0, AT_Q);
     pdl_wait_prior_grids();
 
-    const int h = blockIdx.y, kvh = h / (g.heads / g.kv_heads);
-    const int r0 = blockIdx.x * AT_Q;
     const int pos0 = g.meta[0], slot = g.meta[1];
     const int p0 = pos0 + r0, p1 = min(pos0 + g.rows, p0 + AT_Q) - 1;     // positions of the CTA's first and last query
     int sinks, lo;

@@ -78,7 +78,16 @@ struct AttnArgs {
     const int* meta;
     int ld, gate_off;           // gate_off < 0: no output gate
     int heads, kv_heads, dim_pad, vdim_pad, window, keep_first, capacity, bias_len, rows;
+    int first_pos;              // meta[0] as the host knows it: what may be asked for before the kernel ahead has ended
     float scale;
+
+    // The biases of the distances that queries r0 ... r0 + n - 1 of a head meet in their window, towards L2: a constant that the layers'
+    // weights drive out from one prompt to the next (100 queries, 16 heads, in a prompt step: 12 -> 9.6 us).
+    __device__ __forceinline__ void prefetch_bias(int h, int r0, int n) const {
+        if (bias_table == nullptr) return;
+        const int farthest = min(min(first_pos + r0 + n, window + n + 128), bias_len);       // tiles start up to 127 keys ahead of the window
+        for (int d = threadIdx.x * 32; d < farthest; d += blockDim.x * 32) l2_prefetch(bias_table + (size_t)h * bias_len + d);
+    }
 };
 
 // One query of one head per CTA: scores one key per thread, 128 keys at a time, then P.V with threads along vdim
