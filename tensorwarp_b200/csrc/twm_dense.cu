@@ -7,6 +7,7 @@
 #include <unordered_map>
 
 #include "twm_dense_attn.cuh"
+#include "twm_dense_attn_f32.cuh"
 #include "twm_dense_attn_tc.cuh"
 #include "twm_dense_common.cuh"
 #include "twm_dense_decode.cuh"
@@ -687,6 +688,21 @@ twm_status attention_tc(const AttnArgs<bf16>& g, int end, int slots, int flags, 
 }
 twm_status attention_tc(const AttnArgs<float>&, int, int, int, void*) { return invalid("the tcgen05 attention takes bfloat16"); }
 
+// The FP32 attention of several queries to a CTA: one query a warp while that leaves SMs idle (70 queries, 16 heads: 144 CTAs), else four.
+bool attention_f32_fits(const AttnArgs<bf16>&) { return false; }
+bool attention_f32_fits(const AttnArgs<float>& g)
+{
+    return g.vdim_pad <= 128 && attn_f32_smem_bytes(g.dim_pad, g.vdim_pad, 4) <= kSmemLimit && g.ld % 4 == 0 && ((uintptr_t)g.proj & 15) == 0 &&
+           ((uintptr_t)g.k_cache & 15) == 0 && ((uintptr_t)g.v_cache & 15) == 0 && ((uintptr_t)g.out & 15) == 0;
+}
+twm_status attention_f32(const AttnArgs<bf16>&, int, int, void*) { return invalid("the FP32 attention takes float"); }
+twm_status attention_f32(const AttnArgs<float>& g, int sms, int flags, void* stream)
+{
+    const int nq = (long)g.rows * g.heads > 2L * AF_WARPS * 4 * sms ? 4 : 1, per = AF_WARPS * nq;
+    return launch("attn_f32", nq == 4 ? attn_f32_kernel<4> : attn_f32_kernel<1>, dim3((g.rows + per - 1) / per, g.heads), AF_THREADS,
+                  attn_f32_smem_bytes(g.dim_pad, g.vdim_pad, nq), flags, stream, 0, g);
+}
+
 template <typename T>
 twm_status attention(const twm_dense_model* m, const twm_dense_layer& l, const twm_dense_buffers* b, int rows, int first_pos,
                      int kernel, int flags, void* stream)
@@ -697,6 +713,11 @@ twm_status attention(const twm_dense_model* m, const twm_dense_layer& l, const t
     if (kernel == 3 || (kernel == 0 && attention_tc_fits(g))) return attention_tc(g, first_pos + rows, m->slots, flags, stream);
     if (kernel == 2 && !attention_tiles_fit(g)) return invalid("the tensor-core attention takes bfloat16 heads that fit shared memory");
     if (kernel == 2 || (kernel == 0 && attention_tiles_fit(g))) return attention_tiles(g, flags, stream);
+    if (kernel == 0 && attention_f32_fits(g)) {
+        int sms = 148;
+        TRY(device(&sms));
+        return attention_f32(g, sms, flags, stream);
+    }
     const int vblock = AS_VPT * AS_THREADS;
     return launch("attn_simt", attn_simt_kernel<T>, dim3(rows, l.heads, (l.vdim_pad + vblock - 1) / vblock), AS_THREADS,
                   sizeof(float) * (size_t)(l.dim_pad + AS_THREADS), flags, stream, 0, g);

@@ -1,5 +1,6 @@
 """GPU tests of prompt steps at the sizes where their kernels share the work out differently: rows of several tokens to a CTA, tiles of 224 and
-192 columns on a pair of SMs."""
+192 columns on a pair of SMs, FP32 attention of several queries to a CTA."""
+import ctypes as C
 import math
 
 import pytest
@@ -63,3 +64,29 @@ def test_tiles_on_a_pair_of_sms(m, n, k, epi):
         ref = gelu_tanh(ref[:, :n]) * ref[:, n:]
     bound = ref.abs() * (2 ** -8 if epi != _dense.EPI_STORE_F32 else 1e-5) + 3e-5      # as test_gemm: one rounding, sums of K FP32 terms
     assert bool(((got - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,window,keep", [(4, 2, 64, 64, 64, 1), (16, 1, 128, 128, 65, 64), (2, 2, 48, 96, None, 0), (3, 3, 160, 112, 1, 5),
+                                                                 (64, 4, 32, 16, 33, 40)])
+@pytest.mark.parametrize("first,rows", [(0, 1), (0, 7), (5, 70), (0, 200), (190, 33)])
+def test_f32_attention_equals_one_query_to_a_cta(heads, kv_heads, dim, vdim, window, keep, first, rows):
+    """The same bits as kernel 1, also where keys that a query does not see hold values that are not numbers."""
+    cfg = bidasun_cases.config(64, 50, [bidasun_cases.layer(bidasun_cases.attention(heads, kv_heads, dim, vdim, window, keep), None)])
+    eng = bidasun_engine(cfg, torch.float32, max_live=2)
+    seq = eng.open()
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    eng._buf["proj"].normal_(generator=gen)
+    for cache in (eng.state.k[0], eng.state.v[0]):
+        cache.normal_(generator=gen)
+        cache[:, first + rows - 1:] = float("nan")                       # the last query's key, seen by no other
+    out = []
+    for kernel in (1, 0):
+        eng._buf["att"].fill_(7.0)
+        torch.cuda.synchronize()
+        eng._set_step(first, seq)
+        _dense.check(_dense.lib().twm_dense_attention(C.byref(eng._desc), 0, C.byref(eng._b), rows, first, kernel, 0, eng.stream.cuda_stream), "attention")
+        eng.stream.synchronize()
+        out.append(eng._buf["att"].clone())
+    assert torch.equal(out[0][:rows - 1], out[1][:rows - 1]) and bool(torch.isfinite(out[0][:rows - 1]).all())
+    assert torch.equal(out[0].isnan(), out[1].isnan()) and bool((out[1][rows:] == 7.0).all())
+    assert _dense.device_error() == 0
