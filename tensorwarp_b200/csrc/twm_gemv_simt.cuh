@@ -131,19 +131,14 @@ gemv_kernel(const GemmParams p)
                 }
                 __syncwarp();
             }
-            if (lane == 0) {
-                mbar_arrive_expect_tx(&sm.full[slot], tx);
-                for (int r = 0; r < nb; ++r) {
-                    bulk_g2s(&sm.packed[slot][r * NT * kBlockBytes],
-                             packed + ((size_t)(bstart + r) * p.N + n0) * kBlockBytes,
-                             (uint32_t)cols * kBlockBytes, &sm.full[slot]);
-                }
-                if (scale_bulk_ok) {
-                    for (int r = 0; r < nrows; ++r) {
-                        bulk_g2s(&sm.scales[slot][r][0], scales + (size_t)(srow_first + r) * p.N + n0,
-                                 (uint32_t)cols * 2, &sm.full[slot]);
-                    }
-                }
+            if (lane == 0) mbar_arrive_expect_tx(&sm.full[slot], tx);
+            __syncwarp();
+            if (lane < nb) {                                        // a lane a row: one after the other, sixteen copies take a third of a microsecond
+                bulk_g2s(&sm.packed[slot][lane * NT * kBlockBytes], packed + ((size_t)(bstart + lane) * p.N + n0) * kBlockBytes,
+                         (uint32_t)cols * kBlockBytes, &sm.full[slot]);
+            } else if (scale_bulk_ok && lane >= 16 && lane - 16 < nrows) {
+                const int r = lane - 16;
+                bulk_g2s(&sm.scales[slot][r][0], scales + (size_t)(srow_first + r) * p.N + n0, (uint32_t)cols * 2, &sm.full[slot]);
             }
             __syncwarp();
         }
@@ -174,22 +169,30 @@ gemv_kernel(const GemmParams p)
         {
             const size_t kbase = (size_t)(b0 + chunk0) * kBlockK;
             const int limit = MMAX * chunk_k;
-            for (int idx = tid; idx < limit; idx += CONSUMERS) {
-                const int m = idx / chunk_k;
-                const int kk = idx - m * chunk_k;
-                float v = 0.0f;
-                if (m < p.M) {
-                    const size_t off = (size_t)m * p.lda + kbase + kk;
-                    v = p.a_is_f16 ? __half2float(reinterpret_cast<const __half*>(p.a)[off])
-                                   : reinterpret_cast<const float*>(p.a)[off];
-                }
-                const int j = kk & 7;
-                const int bitpos = (j < 6) ? 4 * j : 4 * j - 8;
-                sm.a[idx] = v * as_f32((uint32_t)(127 + PRESCALE_EXP - bitpos) << 23);
-                float s = v;
+            constexpr int AHEAD = 4;                                // a thread's values that are asked for before the first is used
+            for (int base = tid; base < limit; base += AHEAD * CONSUMERS) {
+                float v[AHEAD];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (lane == 0) sm.asum8[idx >> 5] = -8.0f * s;
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int idx = base + u * CONSUMERS, m = MMAX == 1 ? 0 : idx / chunk_k;
+                    v[u] = 0.0f;
+                    if (idx < limit && m < p.M) {
+                        const size_t off = (size_t)m * p.lda + kbase + (idx - m * chunk_k);
+                        v[u] = p.a_is_f16 ? __half2float(reinterpret_cast<const __half*>(p.a)[off]) : reinterpret_cast<const float*>(p.a)[off];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int idx = base + u * CONSUMERS;           // whole blocks of 32: a warp is in or out
+                    if (idx >= limit) break;
+                    const int j = idx & 7;
+                    const int bitpos = (j < 6) ? 4 * j : 4 * j - 8;
+                    sm.a[idx] = v[u] * as_f32((uint32_t)(127 + PRESCALE_EXP - bitpos) << 23);
+                    float s = v[u];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                    if (lane == 0) sm.asum8[idx >> 5] = -8.0f * s;
+                }
             }
         }
         named_bar_sync(1, CONSUMERS);
