@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 # TWMARLIN_LIB points at another build of the same library (e.g. one compiled with other tuning macros)
@@ -34,6 +35,12 @@ class GemmArgs(C.Structure):
         ("a_prologue", C.c_int),
         ("next", C.c_void_p),
     ]
+
+
+# the same structure as bytes, from all fields in order (pointers as integers, 0 = null)
+_gemm_args = struct.Struct("@6iPlPPPlPN3iPPiPiP")
+assert _gemm_args.size == C.sizeof(GemmArgs)
+pack_gemm_args = _gemm_args.pack
 
 
 class Comm(C.Structure):
@@ -77,7 +84,7 @@ class Plan(C.Structure):
 SIGNATURES = {
     "twm_plan": (C.c_int, [C.c_int] * 7 + [C.POINTER(Plan)]),
     "twm_workspace_bytes": (C.c_size_t, [C.c_int] * 4),
-    "twm_gemm_w4a16": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p]),
+    "twm_gemm_w4a16": (C.c_int, [C.c_void_p, C.c_void_p]),              # a twm_gemm_args by reference, or as bytes
     "twm_gemm_w4a16_static_ws": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p]),
     "twm_static_ws_capacity": (C.c_size_t, []),
     "twm_moe_workspace_bytes": (C.c_size_t, [C.c_int] * 4),

@@ -28,6 +28,7 @@ from ._lib import GemmArgs, Plan, TwmError, check
 BLOCK_SIZE = 32  # quantize.rs:25
 
 _DTYPES = {torch.float32: _lib.TWM_F32, torch.float16: _lib.TWM_F16}
+_SCALE_DTYPES = frozenset((torch.float16, torch.uint16, torch.int16))
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
@@ -89,10 +90,14 @@ def gemm_tw_marlin(a: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, 
     (2k values) and the GEMM reads silu(gate) * up: fused_silu_mul (ops.rs:966-977) without its pass.
     ``next_gemm=(packed, scales, m, n, k, group_size)`` names the GEMM that follows on the stream (same
     dtypes and workspace): while this one drains, the head of that one's weights is pulled into L2."""
-    _require_cuda(a, packed, scales, c)
-    if a.dtype not in _DTYPES or c.dtype not in _DTYPES:
+    # This runs once per product, and a product of one row takes no longer than its call: every attribute is read once, and the
+    # arguments are packed by struct, not field by field (5.1 -> 3.4 us of Python a call; one FP32 row through four products 31.1 -> 28.9).
+    if not (a.is_cuda and packed.is_cuda and scales.is_cuda and c.is_cuda):
+        _require_cuda(a, packed, scales, c)
+    a_dtype, c_dtype = _DTYPES.get(a.dtype), _DTYPES.get(c.dtype)
+    if a_dtype is None or c_dtype is None:
         raise TwmError(_lib.TWM_EINVAL, "gemm_tw_marlin: A and C must be float32 or float16")
-    if packed.dtype != torch.uint8 or scales.dtype not in (torch.float16, torch.uint16, torch.int16):
+    if packed.dtype is not torch.uint8 or scales.dtype not in _SCALE_DTYPES:
         raise TwmError(_lib.TWM_EINVAL, "gemm_tw_marlin: packed must be uint8 and scales float16")
     a_cols = k if a_prologue == _lib.TWM_A_PLAIN else 2 * k
     if a.numel() < m * a_cols or c.numel() < m * n:
@@ -100,27 +105,21 @@ def gemm_tw_marlin(a: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, 
     if packed_offsets is None:
         if packed.numel() < (k // 32) * n * 16 or scales.numel() < (k // group_size) * n:
             raise TwmError(_lib.TWM_EINVAL, "gemm_tw_marlin: packed or scales smaller than the stated shape")
-    lda = a.stride(0) if a.dim() == 2 else a_cols
-    ldc = c.stride(0) if c.dim() == 2 else n
-    args = GemmArgs(
-        M=m, N=n, K=k, group_size=group_size,
-        a_dtype=_DTYPES[a.dtype], c_dtype=_DTYPES[c.dtype],
-        a=a.data_ptr(), lda=lda, packed=packed.data_ptr(), scales=scales.data_ptr(),
-        c=c.data_ptr(), ldc=ldc,
-        workspace=workspace.ptr if workspace is not None else None,
-        workspace_bytes=workspace.nbytes if workspace is not None else 0,
-        splits_override=splits_override, kernel_override=kernel_override, flags=flags,
-        packed_offsets=packed_offsets.data_ptr() if packed_offsets is not None else None,
-        scales_offsets=scales_offsets.data_ptr() if scales_offsets is not None else None,
-        expert_idx=expert_idx, a_prologue=a_prologue,
-    )
+    ws_ptr, ws_bytes = (workspace.ptr, workspace.nbytes) if workspace is not None else (0, 0)
+    following = 0
     if next_gemm is not None:
         np_, ns_, nm, nn, nk, ng = next_gemm
-        nxt = GemmArgs(M=nm, N=nn, K=nk, group_size=ng, a_dtype=args.a_dtype, c_dtype=args.c_dtype,
-                       packed=np_.data_ptr(), scales=ns_.data_ptr(), workspace=args.workspace,
-                       workspace_bytes=args.workspace_bytes)
-        args.next = C.addressof(nxt)          # read during the call below only
-    check(_lib.lib().twm_gemm_w4a16(C.byref(args), _stream_ptr(stream)), "twm_gemm_w4a16")
+        nxt = GemmArgs(M=nm, N=nn, K=nk, group_size=ng, a_dtype=a_dtype, c_dtype=c_dtype,
+                       packed=np_.data_ptr(), scales=ns_.data_ptr(), workspace=ws_ptr, workspace_bytes=ws_bytes)
+        following = C.addressof(nxt)          # read during the call below only
+    args = _lib.pack_gemm_args(
+        m, n, k, group_size, a_dtype, c_dtype,
+        a.data_ptr(), a.stride(0) if a.dim() == 2 else a_cols, packed.data_ptr(), scales.data_ptr(),
+        c.data_ptr(), c.stride(0) if c.dim() == 2 else n, ws_ptr, ws_bytes, splits_override, kernel_override, flags,
+        packed_offsets.data_ptr() if packed_offsets is not None else 0,
+        scales_offsets.data_ptr() if scales_offsets is not None else 0,
+        expert_idx, 0, a_prologue, following)
+    check(_lib.lib().twm_gemm_w4a16(args, _stream_ptr(stream)), "twm_gemm_w4a16")
 
 
 def gemm_tw_marlin_m1(a: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, c: torch.Tensor,
