@@ -978,7 +978,11 @@ twm_status gemv(GemvArgs<T> g, int sms, int flags, void* stream)
     const size_t act = gemv_smem_bytes(row_bytes, parts, 0), limit = kSmemLimit - 8 * 1024;      // static shared memory beside it
     if (act + 2 * GV_STAGE > limit) return invalid("an input row does not fit shared memory");
     g.stages = (int)std::min<size_t>(GV_MAX_STAGES, (limit - act) / GV_STAGE);
-    return launch("gemv", gemv_kernel<T, PRO, EPI, ROUTE>, dim3(grid), GV_THREADS, gemv_smem_bytes(row_bytes, parts, g.stages), flags, stream, 0, g);
+    auto kernel = gemv_kernel<T, PRO, EPI, ROUTE, 4>;
+    if constexpr (PRO != PRO_VEC) {
+        if (g.src.wp <= 2 * 4 * GV_CONSUMERS) kernel = gemv_kernel<T, PRO, EPI, ROUTE, 2>;
+    }
+    return launch("gemv", kernel, dim3(grid), GV_THREADS, gemv_smem_bytes(row_bytes, parts, g.stages), flags, stream, 0, g);
 }
 
 // --------------------------------------------- one decoded token's mixers --
@@ -997,11 +1001,12 @@ twm_status sigmoid_decode(const twm_dense_model* m, const twm_dense_layer& l, co
     const long visible = std::min<long>((long)l.window + l.keep_first, m->capacity);
     int splits = 1;
     while (splits < 16 && visible > 64L * splits && l.kv_heads * splits * 2 <= sms) splits *= 2;
-    // a chunk of keys and values that leaves room for a product's CTA on the same SM, where heads are not too wide
+    // a chunk of keys and values that holds a CTA's share, but leaves room for a product's CTA on the same SM, where heads are not too wide
+    const long share = (visible + splits - 1) / splits;
     auto bytes = [&](int chunk) { return attn_decode_smem_bytes<T>(l.heads / l.kv_heads, l.dim_pad, l.vdim_pad, chunk, splits); };
     t.parts = attn_decode_parts(l.heads / l.kv_heads, l.vdim_pad);
-    t.chunk = AD_MAX_CHUNK;
-    while (t.chunk > 8 && bytes(t.chunk) > 80 * 1024) t.chunk /= 2;
+    t.chunk = (int)std::min<long>(AD_MAX_CHUNK, (share + 7) / 8 * 8);
+    while (t.chunk > 8 && bytes(t.chunk) > 60 * 1024) t.chunk = (t.chunk / 2 + 7) / 8 * 8;
     return launch("attn_decode", attn_decode_kernel<T>, dim3(splits, l.kv_heads), AD_THREADS, bytes(t.chunk), flags, stream, splits, t);
 }
 

@@ -73,7 +73,8 @@ __host__ __device__ inline size_t gemv_smem_bytes(size_t row_bytes, int parts, i
     return (size_t)stages * GV_STAGE + (parts > 1 ? (size_t)parts * gemv_pieces(row_bytes) * GV_PIECE : ((row_bytes + 127) & ~(size_t)127));
 }
 
-template <typename T, int PRO, int EPI, int ROUTE>
+// PER: vectors of a residual row that a thread holds (of rows of up to PER * 1024 columns).
+template <typename T, int PRO, int EPI, int ROUTE, int PER>
 __global__ void __launch_bounds__(GV_THREADS, 1)
 gemv_kernel(const __grid_constant__ GemvArgs<T> g)
 {
@@ -166,6 +167,30 @@ gemv_kernel(const __grid_constant__ GemvArgs<T> g)
     }
 
     // ------------------------------------------------------- prologue (256 threads) --
+    // The factors of the norms and of the shift are constants that a token's weights drive out of L2: asked for while the kernel before runs,
+    // into registers where a row is narrow (of wider ones they would keep the mixer behind this launch from starting beside it: a
+    // latent_decode_kernel of 12.3 us took 15.0), else towards L2.  A prompt of 37 tokens and 24 decoded ones, 16 layers 2048 wide: 15.55 ms
+    // without this and attn_decode_kernel's hints, 14.75 ms with both; on linear and latent layers with experts 19.98 and 19.60.
+    constexpr bool JOINS = ROUTE == ROUTE_NONE && PRO != PRO_VEC, AHEAD = JOINS && PER <= 2;
+    const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+    const float* factor_row = PRO == PRO_SHIFT ? g.shift : PRO == PRO_NORM ? g.pre_norm : nullptr;
+    auto norm_at = [&](int i) { return g.src.y_norm != nullptr ? __ldg(reinterpret_cast<const float4*>(g.src.y_norm) + i) : one; };
+    auto factor_at = [&](int i) { return factor_row != nullptr ? __ldg(reinterpret_cast<const float4*>(factor_row) + i) : one; };
+    float4 norms[AHEAD ? PER : 1], factors[AHEAD ? PER : 1];
+    if (AHEAD) {
+#pragma unroll
+        for (int j = 0; j < (AHEAD ? PER : 1); ++j) {
+            const int i = tid + j * GV_CONSUMERS;
+            const bool in = i < (g.src.wp >> 2);
+            norms[j] = in ? norm_at(i) : one;
+            factors[j] = in ? factor_at(i) : one;
+        }
+    } else if (JOINS) {
+        for (int i = tid * 32; i < g.src.wp; i += GV_CONSUMERS * 32) {
+            if (g.src.y_norm != nullptr) l2_prefetch(g.src.y_norm + i);
+            if (factor_row != nullptr) l2_prefetch(factor_row + i);
+        }
+    }
     pdl_wait_prior_grids();
     if (ROUTE == ROUTE_ROWS) pdl_launch_dependents();
     if (ROUTE == ROUTE_COLUMNS) {
@@ -187,25 +212,24 @@ gemv_kernel(const __grid_constant__ GemvArgs<T> g)
         float* st = PRO == PRO_SHIFT ? g.shift_state + (size_t)g.meta[1] * 2 * wp : nullptr;
         const float* st_before = PRO == PRO_SHIFT && pos > 0 ? st + (size_t)((pos - 1) & 1) * wp : nullptr;
         float fr = 1.0f;
-        // element i of the residual row x; before = the state's, for the token shift
-        auto finish = [&](int i, const float4 x, const float4 before) {
+        // element i of the residual row x; before = the state's, for the token shift; factor = the shift's or the norm's
+        auto finish = [&](int i, const float4 x, const float4 before, const float4 factor) {
             float4 h = x;
             if (PRO == PRO_SHIFT) {
-                h = shift4(x, before, __ldg(reinterpret_cast<const float4*>(g.shift) + i));
+                h = shift4(x, before, factor);
                 if (writer) reinterpret_cast<float4*>(st + (size_t)(pos & 1) * wp)[i] = x;      // the other half of the pair
             }
-            if (PRO == PRO_NORM) h = scale4(x, fr, __ldg(reinterpret_cast<const float4*>(g.pre_norm) + i));
+            if (PRO == PRO_NORM) h = scale4(x, fr, factor);
             if (writer && g.x_out != nullptr) reinterpret_cast<float4*>(g.x_out)[i] = x;
             store4<T>(as + i * 4, h);
         };
         auto state_at = [&](int i) {
             return st_before != nullptr ? reinterpret_cast<const float4*>(st_before)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         };
-        constexpr int PER = 4;
         // without a norm of its own the input is taken this way only where nothing but a normed sublayer output joins
         const bool plain = g.src.y != nullptr && g.src.y_norm != nullptr && g.src.step == nullptr;
         if (nvec <= PER * GV_CONSUMERS && g.src.tokens == nullptr && (PRO == PRO_NORM || plain)) {
-            // rows of up to 4096: everything is requested before the first use
+            // everything is requested before the first use
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 x[PER], y[PER], before[PER];
 #pragma unroll
@@ -228,8 +252,7 @@ gemv_kernel(const __grid_constant__ GemvArgs<T> g)
             for (int j = 0; j < PER; ++j) {
                 const int i = tid + j * GV_CONSUMERS;
                 if (i < nvec) {
-                    float4 n = make_float4(1.f, 1.f, 1.f, 1.f);
-                    if (normed) n = __ldg(reinterpret_cast<const float4*>(g.src.y_norm) + i);
+                    const float4 n = !normed ? one : AHEAD ? norms[AHEAD ? j : 0] : norm_at(i);
                     x[j].x += y[j].x * ir * n.x; x[j].y += y[j].y * ir * n.y; x[j].z += y[j].z * ir * n.z; x[j].w += y[j].w * ir * n.w;
                     if (PRO == PRO_NORM && g.src.step != nullptr) {
                         const float4 t = __ldg(reinterpret_cast<const float4*>(g.src.step) + i);
@@ -241,7 +264,7 @@ gemv_kernel(const __grid_constant__ GemvArgs<T> g)
             if (PRO == PRO_NORM) fr = inv_rms(group_sum(ss, red, GV_CONSUMERS, 1), g.src.width, g.src.eps);
 #pragma unroll
             for (int j = 0; j < PER; ++j)
-                if (tid + j * GV_CONSUMERS < nvec) finish(tid + j * GV_CONSUMERS, x[j], before[j]);
+                if (tid + j * GV_CONSUMERS < nvec) finish(tid + j * GV_CONSUMERS, x[j], before[j], AHEAD ? factors[AHEAD ? j : 0] : factor_at(tid + j * GV_CONSUMERS));
         } else {
             const float ir = g.src.row_inv_rms(0, red, GV_CONSUMERS, 1);
             if (PRO == PRO_NORM) {
@@ -249,7 +272,7 @@ gemv_kernel(const __grid_constant__ GemvArgs<T> g)
                 for (int i = tid; i < nvec; i += GV_CONSUMERS) ss += ops::sumsq4(g.src.at(0, pos, tok, i, ir));
                 fr = inv_rms(group_sum(ss, red, GV_CONSUMERS, 1), g.src.width, g.src.eps);
             }
-            for (int i = tid; i < nvec; i += GV_CONSUMERS) finish(i, g.src.at(0, pos, tok, i, ir), state_at(i));
+            for (int i = tid; i < nvec; i += GV_CONSUMERS) finish(i, g.src.at(0, pos, tok, i, ir), state_at(i), factor_at(i));
         }
     }
     named_bar_sync(1, GV_CONSUMERS);
@@ -474,8 +497,10 @@ __host__ inline size_t attn_decode_smem_bytes(int group, int dim_pad, int vdim_p
            (size_t)chunk * (dim_pad * sizeof(T) + 16 + vdim_pad * sizeof(T));
 }
 
+// (The bound is on registers, 80 a thread: with a small share of keys in shared memory, a CTA of the product behind it starts on the same SM
+// and streams its weights meanwhile.  Without it, 126 registers, 6.7 us of a decoded token's layer; with 64, 8.5.)
 template <typename T>
-__global__ void __launch_bounds__(AD_THREADS)
+__global__ void __launch_bounds__(AD_THREADS + 256)
 attn_decode_kernel(const AttnDecodeArgs<T> g)
 {
     using V = Vec<T>;
@@ -506,6 +531,28 @@ attn_decode_kernel(const AttnDecodeArgs<T> g)
         nq[j] = g.q_norm != nullptr && i < group * g.dim_pad ? __ldg(g.q_norm + kvh * group * g.dim_pad + i) : 1.0f;
     }
     const float nk = g.k_norm != nullptr && tid < g.dim_pad ? __ldg(g.k_norm + kvh * g.dim_pad + tid) : 1.0f;
+    // This share's cached rows and biases, which a token's weights have driven out of L2, towards it while the product before runs: a hint,
+    // for the position may still be that of the token before.
+    {
+        const volatile int* meta = g.meta;
+        const int p = meta[0], slot = meta[1];
+        int sinks, lo;
+        visible_range(p, g.window, g.keep_first, sinks, lo);
+        const int total = sinks + (p - lo + 1), per = (total + splits - 1) / splits, first = rank * per, n = min(per, total - first);
+        constexpr int LINE = 128 / sizeof(T);
+        const int kl = (g.dim_pad + LINE - 1) / LINE, vl = (g.vdim_pad + LINE - 1) / LINE;
+        for (int i = tid; i < n * (kl + vl); i += AD_THREADS) {
+            const int r = i / (kl + vl), c = i - r * (kl + vl), t = first + r, j = t < sinks ? t : lo + (t - sinks);
+            if (j >= 0 && j < g.capacity)
+                l2_prefetch(c < kl ? g.k_cache + ((size_t)slot * g.capacity + j) * kd + kvh * g.dim_pad + c * LINE
+                                   : g.v_cache + ((size_t)slot * g.capacity + j) * vd + kvh * g.vdim_pad + (c - kl) * LINE);
+        }
+        if (g.bias_table != nullptr && n > 0)
+            for (int i = tid; i < group * 8; i += AD_THREADS) {                    // distances of the share's last keys: eight lines a head
+                const int h = i >> 3, j = (first + n - 1) < sinks ? first + n - 1 : lo + (first + n - 1 - sinks), d = p - j + (i & 7) * 32;
+                if (d >= 0 && d < g.bias_len && (i & 7) * 32 < n + 32) l2_prefetch(g.bias_table + (size_t)(kvh * group + h) * g.bias_len + d);
+            }
+    }
     pdl_wait_prior_grids();
     const int p = g.meta[0], slot = g.meta[1];
     // everything of the projection that is needed is asked for before the first use: the newest key and value, the sums of the norms
