@@ -851,6 +851,18 @@ twm_status routed_ff(const twm_dense_model* m, const twm_dense_layer& l, const t
                            l.ff_pad, TWM_EPI_STORE, 0, flags, stream);
 }
 
+template <typename T, int PRO, int EPI = TWM_EPI_STORE_F32, int ROUTE = ROUTE_NONE>
+twm_status gemv(GemvArgs<T> g, int sms, int flags, void* stream);
+
+// The head of one FP32 row: the streaming product, where the row fits (32768 x 2048, 268 MB: 74.6 us as a product of up to eight rows, whose
+// loads have no queue ahead of them; 41.4 us this way, 6.5 TB/s).
+bool head_streams(const twm_dense_model*, const bf16*) { return false; }
+bool head_streams(const twm_dense_model* m, const float* a)
+{
+    return ((uintptr_t)a & 15) == 0 && ((uintptr_t)m->head & 15) == 0 &&
+           gemv_smem_bytes(sizeof(float) * (size_t)m->width_pad, 1, GV_MAX_STAGES) <= kSmemLimit - 8 * 1024;
+}
+
 template <typename T>
 twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int rows, int first_pos, int n_want, float* layer_trace,
                    int flags, void* stream)
@@ -952,13 +964,18 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
     if (n_want > 0) {
         TRY(launch("final_rows", final_rows_kernel<T>, dim3(n_want), ROW_THREADS, sizeof(float) * (size_t)wp, flags, stream, 0,
                    source(nullptr), (T*)b->a, m->final_norm, (const int*)b->want, (const int*)b->meta));
+        if (n_want == 1 && head_streams(m, (const T*)b->a)) {
+            GemvArgs<T> g = {};
+            g.w = (const T*)m->head; g.N = m->vocab; g.ldw = wp; g.out = b->logits; g.meta = b->meta; g.vec = (const float*)b->a;
+            return gemv<T, PRO_VEC>(g, sms, flags, stream);
+        }
         TRY(gemm<T>((const T*)b->a, wp, (const T*)m->head, wp, b->logits, m->vocab, n_want, m->vocab, wp, TWM_EPI_STORE_F32, 0,
                     flags, stream));
     }
     return TWM_OK;
 }
 
-template <typename T, int PRO, int EPI = TWM_EPI_STORE_F32, int ROUTE = ROUTE_NONE>
+template <typename T, int PRO, int EPI, int ROUTE>
 twm_status gemv(GemvArgs<T> g, int sms, int flags, void* stream)
 {
     constexpr bool GATED = EPI == TWM_EPI_GELU_GLU;
