@@ -1,6 +1,7 @@
 // twm_dense.cu — host side and C ABI of the dense-weight decoder models (include/twm_dense.h).  A library of
 // its own (libtwmdense.so): a model with 16-bit weights needs none of the 4-bit kernels.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 #include <type_traits>
@@ -21,6 +22,7 @@
 #include "twm_dense_softmax_tc.cuh"
 #include "twm_dense_tc.cuh"
 #include "twm_dense_tc2.cuh"
+#include "twm_dense_experts_tc.cuh"
 #include "twm_dense_tcs.cuh"
 
 namespace {
@@ -317,6 +319,21 @@ twm_status grouped_gemm_tc_launch(const bf16* a, int lda, const bf16* w, int ldw
                   TcCfg<BN>::SMEM_BYTES, flags, stream, 0, g);
 }
 
+template <int EPI>
+twm_status grouped_gemm_pairs_launch(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, const int* offsets, int experts, int rows,
+                                     int N, int K, int sms, int flags, void* stream)
+{
+    TcArgs g;
+    g.c = c; g.ldc = ldc; g.M = rows; g.N = N; g.K = K;
+    g.n_tiles = (N + 2 * TC_BM - 1) / (2 * TC_BM);
+    g.m_tiles = std::min(rows, rows / EX_TOKENS + experts);            // at most
+    g.offsets = offsets; g.experts = experts;
+    if (!rows_map(&g.a_map, a, rows, K, lda, TC_BM) || !rows_map(&g.w_map, w, (long)experts * N, K, ldw, TC_BM))
+        return invalid("cuTensorMapEncodeTiled refused a map of the grouped tcgen05 product");
+    return launch("gemm_tc2(grouped)", gemm_experts_kernel<EPI>, dim3(2 * (int)std::min<long>(sms / 2, (long)g.m_tiles * g.n_tiles)), TC_THREADS,
+                  Tc2Cfg<EX_TOKENS>::SMEM_BYTES, flags, stream, 2, g);
+}
+
 template <int BN, int EPI>
 twm_status gemm_tc2_launch(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, int M, int N, int K, int sms, int flags,
                            void* stream)
@@ -334,7 +351,8 @@ twm_status gemm_tc2_launch(const bf16* a, int lda, const bf16* w, int ldw, void*
 }
 
 // Tile: the one whose waves cost least.  Measured time of one 64-K stage of a wave: 0.42, 0.25 and 0.20 us for tiles of
-// 128 rows x 256, 128 and 64 columns; 0.33, 0.29 and 0.255 us for 256 x 256, 224 and 192 on a pair of SMs (returned as 512, 448 and 384).
+// 128 rows x 256, 128 and 64 columns; 0.33 us for 256 x 256 on a pair of SMs (returned as 512).  224 and 192 columns (448 and 384) cost in
+// proportion to what they measure beside it: a wave of 72 tiles, K = 8192, one after the other, 54.5, 47.1 and 41.8 us.
 int tc_tile_choice(int M, int N, bool gated, int sms, long* stage_cost)
 {
     int best = 256;
@@ -580,13 +598,36 @@ int grouped_tile_choice(int rows, int experts, int N, int sms)
     }
     return best;
 }
+// Pairs of SMs (twm_dense_experts_tc.cuh) or tiles of `width` columns on one.  A stage of a wave costs 0.42, 0.25 and 0.20 us by width, and 0.33
+// on a pair by the activation rows that it takes, 0.21 at least; an expert's rows end half way through a tile on average.  Up to 96 rows an
+// expert both wait for the weights, and a stage costs what its columns do.  A pair's tiles have to fill the chip once: 16 experts of 512 x 1024,
+// 160 rows each, 16.4 us on 36 pairs and 12.4 on 112 SMs.  Measured, pairs / one SM (rows an expert, evenly 0.7 to 1.3 times): 64 experts of
+// 1024 x 2048: 42 53.5 / 53.0 us, 96 57.4 / 57.1, 128 59.7 / 63.4, 512 129.0 / 137.7; of 2048 x 1024: 42 51.5 / 54.8, 128 57.8 / 61.5, 512
+// 129.9 / 147.8; 32 of 2560 x 3584: 64 114.1 / 112.5, 128 116.7 / 126.5, 512 246.7 / 288.2.
+bool grouped_on_pairs(int rows, int experts, int N, int sms, int width)
+{
+    const int groups = std::min(rows, experts);
+    const double each = (double)rows / groups;
+    const bool streams = each <= 96;
+    auto tiles = [&](int tile_rows, int columns) {
+        return std::ceil(groups * (streams ? 1.0 : std::max(1.0, each / tile_rows + 0.5))) * ((N + columns - 1) / columns);
+    };
+    const double on_pairs = tiles(EX_TOKENS, 2 * TC_BM), taken = each / std::max(1.0, each / EX_TOKENS + 0.5);
+    if (on_pairs < sms / 2) return false;
+    const double stage = streams ? 42.0 * width / 256 : (width == 256 ? 42 : (width == 128 ? 25 : 20));
+    return std::ceil(on_pairs / (sms / 2)) * std::max(21.0, 33 * taken / EX_TOKENS) < std::ceil(tiles(TC_BM, width) / sms) * stage;
+}
 template <int EPI>
 twm_status grouped_gemm_tc(const bf16* a, int lda, const bf16* w, int ldw, void* c, int ldc, const int* offsets, int experts, int rows, int N,
                            int K, int width, int flags, void* stream)
 {
     int sms = 148;
     TRY(device(&sms));
-    if (width == 0) width = grouped_tile_choice(rows, experts, N, sms);
+    if (width == 0) {
+        width = grouped_tile_choice(rows, experts, N, sms);
+        if (grouped_on_pairs(rows, experts, N, sms, width))
+            return grouped_gemm_pairs_launch<EPI>(a, lda, w, ldw, c, ldc, offsets, experts, rows, N, K, sms, flags, stream);
+    }
     switch (width) {
         case 256: return grouped_gemm_tc_launch<256, EPI>(a, lda, w, ldw, c, ldc, offsets, experts, rows, N, K, sms, flags, stream);
         case 128: return grouped_gemm_tc_launch<128, EPI>(a, lda, w, ldw, c, ldc, offsets, experts, rows, N, K, sms, flags, stream);

@@ -90,3 +90,25 @@ def test_f32_attention_equals_one_query_to_a_cta(heads, kv_heads, dim, vdim, win
     assert torch.equal(out[0][:rows - 1], out[1][:rows - 1]) and bool(torch.isfinite(out[0][:rows - 1]).all())
     assert torch.equal(out[0].isnan(), out[1].isnan()) and bool((out[1][rows:] == 7.0).all())
     assert _dense.device_error() == 0
+
+
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_RELU2])
+@pytest.mark.parametrize("counts,n,k,odd", [([0, 1, 255, 256, 257, 0, 31, 33, 1200, 513, 0] * 12, 300, 80, 0), ([300, 0, 0, 224, 225, 161, 96, 1] * 16, 512, 192, 0),
+                                            ([2100, 2, 2303] * 10, 163, 136, 1), ([2100, 2, 2303] * 10, 256, 64, 0), ([42, 0, 1, 127] * 16, 2048, 72, 0),
+                                            ([500, 513, 0, 700] * 4, 1024, 2048, 0)])
+def test_experts_of_many_rows(counts, n, k, odd, epi):
+    """Sizes whose tiles run on pairs of SMs: experts without rows, tiles of 1 to 256 rows, columns past the last whole tile, odd strides."""
+    gen = torch.Generator(device="cuda").manual_seed(n + k)
+    rows, ldc = sum(counts), n + 2 + odd
+    a = torch.randn((rows, k), generator=gen, device="cuda").bfloat16()
+    w = (torch.randn((len(counts), n, k), generator=gen, device="cuda") / math.sqrt(k)).bfloat16()
+    offsets = torch.tensor([sum(counts[:e]) for e in range(len(counts) + 1)], dtype=torch.int32, device="cuda")
+    c = torch.full((rows + 1, ldc), 7.0, dtype=torch.float32 if epi == _dense.EPI_STORE_F32 else torch.bfloat16, device="cuda")
+    _dense.check(_dense.lib().twm_dense_grouped_gemm(_dense.TWM_DENSE_BF16, a.data_ptr(), k, w.data_ptr(), k, c.data_ptr(), ldc, offsets.data_ptr(),
+                                                     len(counts), rows, n, k, epi, 0, 0, torch.cuda.current_stream().cuda_stream), "grouped_gemm")
+    torch.cuda.synchronize()
+    assert _dense.device_error() == 0 and bool((c[:rows, n:] == 7.0).all()) and bool((c[rows] == 7.0).all())
+    want = torch.cat([a[o:o + m].double() @ w[e].double().T for e, (o, m) in enumerate(zip(offsets.tolist(), counts))])
+    if epi == _dense.EPI_RELU2:
+        want = want.clamp(min=0) ** 2
+    assert bool(((c[:rows, :n].double() - want).abs() <= want.abs() * (2 ** -8 if epi != _dense.EPI_STORE_F32 else 2e-5) + 3e-5).all())   # as test_grouped_product
