@@ -518,8 +518,9 @@ twm_status gemm_f32(const float* a, int lda, const float* w, int ldw, void* c, i
     return launch("gemm_f32", gemm_f32_kernel<EPI>, dim3((unsigned)((long)n_tiles * g.splits)), F32_THREADS, F32_SMEM_BYTES, flags, stream,
                   g.splits > 1 ? g.splits : 0, g);
 }
-// From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 5 rows 2.37 / 2.72,
-// 9 rows 2.80 / 2.78, 20 rows 3.33 / 2.88, 70 rows 6.45 / 3.58, 256 rows 18.2 / 8.2; error against 64 bits of 70 rows x 2048 x 8192:
+// From nine rows on the FP32 product runs on the tensor cores.  Prompts of the 1b size, FP32 FMAs / tensor cores, ms: 2 rows 2.28 / 2.31,
+// 5 rows 2.32 / 2.32, 8 rows 2.29 / 2.34; on tensor cores 20 rows 2.39, 70 rows 2.9, 256 rows 5.9 (on FMAs, with attention of one query to a
+// CTA, 3.33, 6.45 and 18.2); error against 64 bits of 70 rows x 2048 x 8192:
 // 4.1e-7 / 1.2e-7.
 // Error against 64 bits over the sum of absolute products (largest, RMS), 70 rows, FP32 FMAs / tensor cores: K = 1 6.0e-8, 2.5e-8 / 8.9e-8,
 // 2.6e-8; K = 2 1.1e-7, 2.6e-8 / 1.5e-7, 2.2e-8; K = 8 1.9e-7, 2.7e-8 / 1.3e-7, 1.5e-8; K = 1024 2.4e-7, 2.8e-8 / 2.7e-8, 4.6e-9: sums of
@@ -943,8 +944,15 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
                    per <= 8 ? residual_rows_kernel<T, 8, F> : residual_rows_kernel<T, 0, F>;
         };
         auto kernel = full ? pick(std::true_type()) : pick(std::false_type());
-        const twm_status st = launch("residual_rows", kernel, dim3((rows + rpc - 1) / rpc), ROW_THREADS,
-                                     per <= 8 ? 0 : sizeof(float) * (size_t)wp, flags, stream, 0, source(next.step), x_next,
+        // One CTA to an SM where there are no more of them, two up to 1.75 times as many (16-bit), by asking for that part of its shared memory.
+        // Started early they gathered on the SMs that were free otherwise, or did not, by how an SM's memory happened to be split: 100 rows, 16
+        // layers 2048 wide, 1 170 or 1 232 us a prompt by the process, now 1 152.  Without / with, us: 30 rows 1 115 / 1 113, 60 1 202 / 1 137, 140
+        // 1 363 / 1 327, 160 1 389 / 1 305, 215 1 421 / 1 371, 250 1 490 / 1 468; not beyond: 20 rows 1 138 / 1 168 (they fit the free SMs), 290
+        // 1 640 / 1 655, and in FP32, whose product leaves no room beside it, 70 2 904 / 2 870 but two to an SM at 160 rows 4 750 / 5 030.
+        const int ctas = (rows + rpc - 1) / rpc;
+        const size_t spread = ctas > sms / 5 && ctas <= sms ? kSmemLimit / 2 + 1024 : sizeof(T) == 2 && ctas > sms && ctas <= sms * 7 / 4 ? kSmemLimit / 3 + 1024 : 0;
+        const twm_status st = launch("residual_rows", kernel, dim3(ctas), ROW_THREADS,
+                                     std::max(spread, per <= 8 ? 0 : sizeof(float) * (size_t)wp), flags, stream, 0, source(next.step), x_next,
                                      want_a ? (T*)b->a : (T*)nullptr, next.shift, next.shift_state, next.pre_norm, b->meta, rows, rpc,
                                      next.clear, next.n_clear);
         std::swap(x, x_next);
