@@ -983,7 +983,9 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
         } else if (l.mixer == TWM_MIX_GLA) {
             TRY(gla_mixer<T>(m, l, b, rows, 0, flags, stream));
         } else {
-            TRY(launch("qk_norm_append", qk_norm_append_kernel<T>, dim3(rows), ROW_THREADS, 0, flags, stream, 0, (T*)b->proj, s.in,
+            // one CTA to an SM, as above: 100 rows 1 160 to 1 246 us a prompt by the process, 1 158 this way; 30 rows 1 110 / 1 131, so from a third on
+            const size_t spread = sizeof(T) == 2 && rows > sms / 3 && rows <= sms ? kSmemLimit / 2 + 1024 : 0;
+            TRY(launch("qk_norm_append", qk_norm_append_kernel<T>, dim3(rows), ROW_THREADS, spread, flags, stream, 0, (T*)b->proj, s.in,
                        l.q_norm, l.k_norm, (T*)l.k_cache, (T*)l.v_cache, s.q, s.k, s.v, l.heads * l.dim, l.kv_heads * l.dim, m->eps,
                        m->capacity, (const float*)x, wp, l.shift ? l.shift_state : (float*)nullptr, b->meta));
             TRY(attention<T>(m, l, b, rows, first_pos, 0, flags, stream));
