@@ -232,10 +232,10 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
     volatile int* abort_flag = &sm.abort_flag;
 
-    // TMA producer state (warp 12).  The first ring-full of stages is issued before the TMEM
+    // TMA producer state (warp 12).  Without wait_first the first ring-full of stages is issued before the TMEM
     // allocation below, so that weights are already streaming while an earlier kernel's CTA may
     // still hold this SM's tensor memory.
     const uint8_t* packed = p.packed;
@@ -274,7 +274,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
     if (warp == WARP_TMA) {
         // ------------------------------ TMA producer (packed, then activations) --
         // Weight stages WSTAGES.. and all activation stages.  Activations come from the
-        // pre-pass kernel, so they wait for the preceding grid; weights never do.
+        // pre-pass kernel, so they wait for the preceding grid; weights do only with wait_first.
         pdl_wait_prior_grids();
         auto issue_b = [&](int st) {
             if (lane == 0) {

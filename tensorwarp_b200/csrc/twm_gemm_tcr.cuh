@@ -100,7 +100,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
     volatile int* abort_flag = &sm.abort_flag;
     if (p.splits > 1) cluster_started();
 
@@ -118,7 +118,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
             bulk_g2s(&sm.sc[(st >> 1) % SSTAGES][0], p.scales + (size_t)((st0 + st) >> 1) * p.N + n0, (uint32_t)NT * 2, &sm.p_full[slot]);
     };
     if (warp == WARP_TMA) {
-        // weights are constants: the first ring-full streams before the preceding kernel has finished
+        // constant weights (without wait_first): the first ring-full streams before the preceding kernel has finished
         if (lane == 0)
             for (int st = 0; st < min(n_stages, PSTAGES); ++st) issue_p(st);
     } else if (warp == WARP_MMA) {

@@ -131,7 +131,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
     volatile int* abort_flag = &sm.abort_flag;
     if (p.cluster_reduce) cluster_started();
 
@@ -147,7 +147,7 @@ gemm_kernel(const __grid_constant__ GemmParams p)
                      &sm.w_full[slot]);
     };
     if (warp == WARP_TMA) {
-        // weights are constants: the first ring-full streams before the preceding kernel has finished
+        // constant weights (without wait_first): the first ring-full streams before the preceding kernel has finished
         if (lane == 0)
             for (int st = 0; st < min(n_stages, WSTAGES); ++st) issue_w(st);
     } else if (warp == WARP_MMA) {

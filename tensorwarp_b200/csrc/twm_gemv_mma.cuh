@@ -707,7 +707,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_launch_dependents();
+    pdl_begin(p.wait_first);
     volatile int* abort_flag = &sm.abort_flag;
 
     float tot[NTL][4];
@@ -717,7 +717,7 @@ gemm_rows_kernel(const __grid_constant__ GemmParams p)
     const int t = lane & 3;
     const int wcol = warp * 16;
     if (warp == CONSUMER_WARPS) {
-        // -------------------------- producer: packed + scales (weights are constants: no wait) --
+        // -------------------------- producer: packed + scales (constants, unless wait_first: no wait of its own) --
         const uint8_t* packed = p.packed;
         const uint16_t* scales = p.scales;
         const bool scale_bulk_ok = ((cols & 7) == 0) && ((p.N & 7) == 0) &&

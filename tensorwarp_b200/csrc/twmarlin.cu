@@ -582,11 +582,11 @@ twm::NextHead next_head_for(const twm_gemm_args* nx, int sm_count)
 }
 
 // How a call's kernels start.  With TWM_FLAG_PDL: beside the kernel before, weights first.  Without: beside it too, but the call's
-// first kernel is idle until that has ended (pdl_begin), which saves the launch latency and promises nothing.  A pre-pass lets the
-// product behind it start only after its own wait, so that product's weights, whatever wrote them, are there.  A call that is being
-// captured keeps plain launches, so that the caller's graph has plain edges.
-// One after the other on a stream, plain launches / this way: four products of 24 rows, 7b layer (eight launches) 86.7 / 69.8 us; of 200
-// rows 190.5 / 172.9; of one FP32 row, 1b layer 38.1 / 32.8; gate/up and down of eight experts 20.5 / 16.2.
+// kernels are idle until that has ended (pdl_begin), the product behind a pre-pass until the pre-pass has, which saves the launch
+// latency and promises nothing.  A call that is being captured keeps plain launches, so that the caller's graph has plain edges.
+// One after the other on a stream, plain launches / this way: four products of 24 rows, 7b layer (eight launches) 86.7 / 69.3 us; of 200
+// rows 190.5 / 176.9; of one FP32 row, 1b layer 38.1 / 32.8; gate/up and down of eight experts 20.5 / 16.2.  A plain launch of the product
+// behind a pre-pass: 24 rows 78.8, 200 rows 187; its first weights asked for towards L2 ahead of the wait: 69.7 and 176.6, as without.
 struct FirstLaunch { int flags; bool wait_first; };
 FirstLaunch first_launch(unsigned flags, cudaStream_t stream)
 {
