@@ -4,7 +4,8 @@
  * through this ABI and captured in one CUDA graph.  Same conventions as twmarlin.h: device
  * pointers owned by the caller, enqueue only, nothing allocated, status returned.  Position and
  * sequence length are read from device buffers (generate.rs:1413-1416), never from launch
- * parameters.  `flags` takes TWM_FLAG_PDL.
+ * parameters.  `flags` takes TWM_FLAG_PDL: the kernels start beside the one before and wait for it before
+ * they read anything that they use, gamma and bias included; no argument needs to be a constant.
  */
 #ifndef TWM_DECODE_H
 #define TWM_DECODE_H

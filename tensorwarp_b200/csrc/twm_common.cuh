@@ -148,6 +148,9 @@ __device__ __forceinline__ void pdl_begin(bool wait_first) {
     pdl_launch_dependents();
 }
 
+// Asks for a line towards L2: a hint, which changes no value that is read later.
+__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
+
 // ------------------------------------------------- thread-block clusters --
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;

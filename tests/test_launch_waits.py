@@ -33,3 +33,11 @@ def test_kernels_of_plain_calls_wait_before_they_read(name):
         assert first is None or at.start() < first.start(), kernel
         # reached by every thread: outside any block but the kernel's own
         assert body[:at.start()].count("{") - body[:at.start()].count("}") == 1, kernel
+
+
+@pytest.mark.parametrize("name,kernel", [("twm_decode_ops.cuh", "rmsnorm_kernel"), ("twm_decode_ops.cuh", "attn_chunk_kernel")])
+def test_factors_and_biases_are_read_after_the_wait(name, kernel):
+    """With TWM_FLAG_PDL too: what the kernel before may write is no more than asked for towards L2 ahead of the wait."""
+    body = dict(kernels(name))[kernel]
+    ahead = body[:body.index("pdl_wait_prior_grids();")]
+    assert "l2_prefetch(" in ahead and not re.search(READS + r"|\b(?:gamma|bias)\[", ahead)
