@@ -19,6 +19,11 @@
  * allocated, status returned.  Position and slot are read from device memory (buffers->meta), so a
  * captured decode step serves every position and slot.
  *
+ * `flags` takes TWM_FLAG_PDL: kernels start beside the ones before them, the first beside whatever is ahead of the call
+ * on the stream.  With it, what the model points to is constant: weights, factors of norms and shifts, biases and
+ * tables are read before that work has ended (the caches and states are not), and so are W of twm_dense_gemm and
+ * twm_dense_grouped_gemm.  Leave the flag clear for a call behind work that writes one of them.
+ *
  * Padding.  Every row length a kernel walks is padded by the loader to a multiple of 16 elements
  * (width_pad, dim_pad, vdim_pad, ff_pad) with zero weights, so padded activations are exactly zero.
  */

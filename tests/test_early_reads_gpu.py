@@ -1,11 +1,15 @@
-"""GPU tests of what a kernel may read while the kernel before it runs (TWM_FLAG_PDL): the 4-bit decoder's small kernels read nothing
-that they use, so factors and biases that that kernel writes are seen."""
+"""GPU tests of what a kernel may read while the kernel before it runs (TWM_FLAG_PDL).  The 4-bit decoder's small kernels: nothing that they
+use, so factors and biases that that kernel writes are seen.  Steps of dense-weight decoders take the model as constant with the flag
+(include/twm_dense.h), and see what was written without it."""
 import pytest
 import torch
 
-from tensorwarp_b200 import _lib
+import bidasun_cases
+import zukotar_cases
+from tensorwarp_b200 import _dense, _lib
 from tensorwarp_b200 import quantize as q
 from test_launch_order_gpu import operands
+from test_prompt_steps_gpu import BOTH, bidasun_engine, zukotar_engine
 
 pytestmark = pytest.mark.gpu
 PDL = _lib.TWM_FLAG_PDL
@@ -80,3 +84,42 @@ def test_biases_of_the_attention(heads, kv_heads, rows, pos, flags):
                                             hd, at.data_ptr(), length.data_ptr(), max_seq, scratch.data_ptr(), scratch.numel(), flags, sp), "twm_attn_decode_rope")
     agree(writer(bias, 18944), read, [out, k[:, pos], v[:, pos]])
     assert q.device_error() == 0
+
+
+@BOTH
+@pytest.mark.parametrize("step", ["prompt", "decode"])
+@pytest.mark.parametrize("design,width", [("bidasun", 1040), ("bidasun", 3088), ("zukotar", 2048)])
+def test_factors_of_a_step_s_first_kernel(design, width, step, dtype):
+    """The shift or norm factors of a dense-weight decoder's first layer, written by a product on the same stream directly before a step
+    without the flag."""
+    if design == "bidasun":
+        cfg = bidasun_cases.config(width, 99, [bidasun_cases.layer(bidasun_cases.attention(2, 1, 64, 64, 70, 3), 64)])
+        eng, name = bidasun_engine(cfg, dtype, use_pdl=False), "shift"
+    else:
+        cfg = zukotar_cases.config(width, 99, [zukotar_cases.layer(zukotar_cases.latent(2, 32, 16, 32, 32, 70), zukotar_cases.experts(2, 2, 32))])
+        eng, name = zukotar_engine(cfg, 16, dtype, max_tokens=320, use_pdl=False), "pre1"
+    factors, lib, rows, k = eng.model.layers[0][name], _dense.lib(), 1 if step == "decode" else 9, 8192
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    sets = [(torch.randn((1, k), generator=gen, device="cuda").to(dtype), (torch.randn((factors.numel(), k), generator=gen, device="cuda") / 90).to(dtype)) for _ in range(2)]
+    for a, w in sets:
+        w[cfg["width"]:] = 0                                              # padding columns stay zero
+    kind = {torch.float32: _dense.TWM_DENSE_F32, torch.bfloat16: _dense.TWM_DENSE_BF16}[dtype]
+    seq = eng.open()
+    toks = bidasun_cases.tokens(cfg, rows, 1)
+    eng._buf["tokens"][:rows].copy_(torch.tensor(toks, dtype=torch.int32))
+    eng._buf["want"][:1].fill_(rows - 1)
+    torch.cuda.synchronize()
+
+    def write(i):
+        a, w = sets[i % 2]
+        eng._set_step(0, seq, toks[0])
+        _dense.check(lib.twm_dense_gemm(kind, a.data_ptr(), k, w.data_ptr(), k, factors.data_ptr(), factors.numel(), 1, factors.numel(), k, _dense.EPI_STORE_F32, 0,
+                                        _dense.TWM_FLAG_PDL, eng.stream.cuda_stream), "gemm")
+
+    def read(i):
+        if step == "decode":
+            eng._enqueue_decode("logits")
+        else:
+            eng.enqueue_prefill(rows, 0, 1)
+    agree(write, read, [eng.logits[:1]])
+    assert _dense.device_error() == 0
