@@ -1069,12 +1069,13 @@ twm_status sigmoid_decode(const twm_dense_model* m, const twm_dense_layer& l, co
     const long visible = std::min<long>((long)l.window + l.keep_first, m->capacity);
     int splits = 1;
     while (splits < 16 && visible > 64L * splits && l.kv_heads * splits * 2 <= sms) splits *= 2;
-    // a chunk of keys and values that holds a CTA's share, but leaves room for a product's CTA on the same SM, where heads are not too wide
+    // a chunk of keys and values that holds a CTA's share, but leaves room for a product's CTA on the same SM, where heads are not too wide (FP32,
+    // 40 heads of 128, us a token at 600 and 2500 tokens: up to 80 KB 1 357 and 1 432, up to 60 KB 1 382 and 1 479)
     const long share = (visible + splits - 1) / splits;
     auto bytes = [&](int chunk) { return attn_decode_smem_bytes<T>(l.heads / l.kv_heads, l.dim_pad, l.vdim_pad, chunk, splits); };
     t.parts = attn_decode_parts(l.heads / l.kv_heads, l.vdim_pad);
     t.chunk = (int)std::min<long>(AD_MAX_CHUNK, (share + 7) / 8 * 8);
-    while (t.chunk > 8 && bytes(t.chunk) > 60 * 1024) t.chunk = (t.chunk / 2 + 7) / 8 * 8;
+    while (t.chunk > 8 && bytes(t.chunk) > 80 * 1024) t.chunk = (t.chunk / 2 + 7) / 8 * 8;
     return launch("attn_decode", attn_decode_kernel<T>, dim3(splits, l.kv_heads), AD_THREADS, bytes(t.chunk), flags, stream, splits, t);
 }
 
