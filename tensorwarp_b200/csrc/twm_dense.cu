@@ -945,12 +945,14 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
         };
         auto kernel = full ? pick(std::true_type()) : pick(std::false_type());
         // One CTA to an SM where there are no more of them, two up to 1.75 times as many (16-bit), by asking for that part of its shared memory.
-        // Started early they gathered on the SMs that were free otherwise, or did not, by how an SM's memory happened to be split: 100 rows, 16
-        // layers 2048 wide, 1 170 or 1 232 us a prompt by the process, now 1 152.  Without / with, us: 30 rows 1 115 / 1 113, 60 1 202 / 1 137, 140
-        // 1 363 / 1 327, 160 1 389 / 1 305, 215 1 421 / 1 371, 250 1 490 / 1 468; not beyond: 20 rows 1 138 / 1 168 (they fit the free SMs), 290
-        // 1 640 / 1 655, and in FP32, whose product leaves no room beside it, 70 2 904 / 2 870 but two to an SM at 160 rows 4 750 / 5 030.
+        // Started early they gathered on the SMs that were free otherwise, or did not, by how an SM's memory happened to be split.  Without /
+        // with, us a prompt, L2 cold, 16 layers 2048 wide: 60 rows 1 192 / 1 148, 80 1 205 / 1 136, 100 1 186 to 1 250 by the process / 1 172, 130 1 337
+        // / 1 311, 170 1 391 / 1 323, 215 1 424 / 1 382; 14 layers 3584 wide: 60 2 037 / 2 021, 120 2 162 / 2 192, 200 the same; 6 layers 5120 wide:
+        // 80 1 096 / 1 073, 200 the same.  Not beyond: 20 rows 1 138 / 1 168 (they fit the free SMs), 290 1 640 / 1 655, and in FP32, whose product
+        // leaves no room beside it, 70 2 904 / 2 870 but two to an SM at 160 rows 4 750 / 5 030; nor where nothing starts early.
         const int ctas = (rows + rpc - 1) / rpc;
-        const size_t spread = ctas > sms / 5 && ctas <= sms ? kSmemLimit / 2 + 1024 : sizeof(T) == 2 && ctas > sms && ctas <= sms * 7 / 4 ? kSmemLimit / 3 + 1024 : 0;
+        const size_t spread = !(flags & TWM_FLAG_PDL) ? 0 : ctas > sms / 5 && ctas <= sms ? kSmemLimit / 2 + 1024 :
+                              sizeof(T) == 2 && ctas > sms && ctas <= sms * 7 / 4 ? kSmemLimit / 3 + 1024 : 0;
         const twm_status st = launch("residual_rows", kernel, dim3(ctas), ROW_THREADS,
                                      std::max(spread, per <= 8 ? 0 : sizeof(float) * (size_t)wp), flags, stream, 0, source(next.step), x_next,
                                      want_a ? (T*)b->a : (T*)nullptr, next.shift, next.shift_state, next.pre_norm, b->meta, rows, rpc,
@@ -983,9 +985,9 @@ twm_status prefill(const twm_dense_model* m, const twm_dense_buffers* b, int row
         } else if (l.mixer == TWM_MIX_GLA) {
             TRY(gla_mixer<T>(m, l, b, rows, 0, flags, stream));
         } else {
-            // one CTA to an SM, as above: 100 rows 1 160 to 1 246 us a prompt by the process, 1 158 this way; 30 rows 1 110 / 1 131, so from a third on
-            const size_t spread = sizeof(T) == 2 && rows > sms / 3 && rows <= sms ? kSmemLimit / 2 + 1024 : 0;
-            TRY(launch("qk_norm_append", qk_norm_append_kernel<T>, dim3(rows), ROW_THREADS, spread, flags, stream, 0, (T*)b->proj, s.in,
+            // (One CTA to an SM, as above, gains nothing here with a cold L2 (100 rows of 2048 1 175 / 1 165 us a prompt, 120 of 3584 2 183 / 2 164, 80 of
+            // 5120 1 074 / 1 089) and costs 4 to 7 % where short prompts follow one another: 80 of 2048 1 054 / 1 121, 100 of 3584 2 038 / 2 106.)
+            TRY(launch("qk_norm_append", qk_norm_append_kernel<T>, dim3(rows), ROW_THREADS, 0, flags, stream, 0, (T*)b->proj, s.in,
                        l.q_norm, l.k_norm, (T*)l.k_cache, (T*)l.v_cache, s.q, s.k, s.v, l.heads * l.dim, l.kv_heads * l.dim, m->eps,
                        m->capacity, (const float*)x, wp, l.shift ? l.shift_state : (float*)nullptr, b->meta));
             TRY(attention<T>(m, l, b, rows, first_pos, 0, flags, stream));
