@@ -3,6 +3,8 @@ wait for it, so what that one writes, weights included, has to be seen, and what
 import pytest
 import torch
 
+import graph_nodes
+from tensorwarp_b200 import _lib
 from tensorwarp_b200 import quantize as q
 
 pytestmark = pytest.mark.gpu
@@ -156,7 +158,35 @@ def test_experts_behind_what_writes_their_weights_choice_and_factors(hidden, ff,
     agree(8, calls, {"shared": [up_scales, ids, factors, mid, acc], "kept": [acc, mid]})
 
 
-def test_captured_calls_keep_plain_launches():
+def calls_of_all_kernels():
+    """One call on each kernel of the products, and one of the experts."""
+    out = []
+    for m, dtype, group in [(1, torch.float16, 128), (24, torch.float16, 128), (48, torch.float16, 128), (100, torch.float16, 128), (200, torch.float16, 128),
+                            (1, torch.float32, 32)]:
+        a, p, s = operands(m, 1024, 2048, group, dtype, m)
+        c, ws = torch.zeros((m, 2048), dtype=dtype, device="cuda"), q.Workspace(q.workspace_bytes(m, 2048, 1024, group))
+        out.append(lambda a=a, p=p, s=s, c=c, group=group, ws=ws, **kw: q.gemm_tw_marlin(a, p, s, c, a.shape[0], 2048, 1024, group_size=group, workspace=ws, **kw))
+    a, p, s = operands(1, 512, 4 * 256, 128, torch.float16, 9)
+    ids, c = torch.tensor([1.0, 3.0], device="cuda"), torch.zeros((2, 256), dtype=torch.float16, device="cuda")
+    ws = q.Workspace(q.moe_workspace_bytes(2, 256, 512, 128))
+    out.append(lambda **kw: q.batched_marlin_gate_up(a.view(-1), p, s, ids, c, p.numel() // 4, s.numel() // 4, 256, 512, 2, group_size=128, workspace=ws, **kw))
+    return out
+
+
+def test_captured_calls_have_plain_edges():
+    """A call without the flag is a plain node of the caller's graph; with it, its kernels are joined by programmatic edges."""
+    calls = calls_of_all_kernels()
+    for call in calls:
+        call()
+    torch.cuda.synchronize()
+    for flags, plain in ((0, True), (_lib.TWM_FLAG_PDL, False)):
+        nodes, edges = graph_nodes.captured(lambda: [call(flags=flags) for call in calls])
+        assert len(nodes) >= len(calls) + 4 and len(edges) == len(nodes) - 1
+        assert edges == [graph_nodes.EDGE_PLAIN if plain else graph_nodes.EDGE_PROGRAMMATIC] * len(edges)
+    assert q.device_error() == 0
+
+
+def test_captured_calls_give_the_same_results():
     """The same results from a graph, and from a stream, of calls that overwrite their weights in between."""
     m, k, n, group = 24, 1024, 1024, 128
     sets = [operands(m, k, n, group, torch.float16, s) for s in range(2)]

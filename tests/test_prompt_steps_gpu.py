@@ -7,6 +7,7 @@ import pytest
 import torch
 
 import bidasun_cases
+import graph_nodes
 import zukotar_cases
 from tensorwarp_b200 import _dense, dense
 from tensorwarp_b200.engine import DenseEngine
@@ -53,7 +54,7 @@ def test_rows_of_several_tokens_to_a_cta(design, width, dtype):
 
 
 @pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
-@pytest.mark.parametrize("m,n,k", [(2048, 3584, 192), (2041, 3570, 80), (4096, 4096, 64), (4000, 4090, 200), (2048, 1792, 128), (2500, 5000, 72)])
+@pytest.mark.parametrize("m,n,k", [(2048, 3584, 192), (2041, 3570, 80), (4096, 4096, 64), (4000, 4090, 200), (2048, 1792, 128), (2500, 5000, 72), (2500, 2050, 72)])
 def test_tiles_on_a_pair_of_sms(m, n, k, epi):
     gen = torch.Generator(device="cuda").manual_seed(m + n)
     a = torch.randn((m, k), generator=gen, device="cuda").bfloat16()
@@ -64,6 +65,19 @@ def test_tiles_on_a_pair_of_sms(m, n, k, epi):
         ref = gelu_tanh(ref[:, :n]) * ref[:, n:]
     bound = ref.abs() * (2 ** -8 if epi != _dense.EPI_STORE_F32 else 1e-5) + 3e-5      # as test_gemm: one rounding, sums of K FP32 terms
     assert bool(((got - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("epi", [_dense.EPI_STORE, _dense.EPI_STORE_F32, _dense.EPI_GELU_GLU])
+@pytest.mark.parametrize("m,n,k,columns,gated", [(2048, 3584, 192, 224, 224), (2041, 3570, 80, 224, 224), (4096, 4096, 64, 192, 256), (4000, 4090, 200, 192, 256),
+                                                 (2048, 1792, 128, 224, 224), (2500, 5000, 72, 256, 256), (2500, 2050, 72, 192, 192)])
+def test_columns_of_the_tiles_on_a_pair_of_sms(m, n, k, columns, gated, epi):
+    """The sizes above are tiled as that test is meant to have them."""
+    a = torch.zeros((m, k), dtype=torch.bfloat16, device="cuda")
+    w = torch.zeros((2 * n if epi == _dense.EPI_GELU_GLU else n, k), dtype=torch.bfloat16, device="cuda")
+    c = torch.zeros((m, n), dtype=torch.float32 if epi == _dense.EPI_STORE_F32 else torch.bfloat16, device="cuda")
+    names, _ = graph_nodes.captured(lambda: _dense.check(_dense.lib().twm_dense_gemm(_dense.TWM_DENSE_BF16, a.data_ptr(), k, w.data_ptr(), k, c.data_ptr(), n, m, n, k,
+                                                                                    epi, 0, 0, torch.cuda.current_stream().cuda_stream), "gemm"))
+    assert len(names) == 1 and f"gemm_tc2_kernelILi{gated if epi == _dense.EPI_GELU_GLU else columns}E" in names[0]
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,window,keep", [(4, 2, 64, 64, 64, 1), (16, 1, 128, 128, 65, 64), (2, 2, 48, 96, None, 0), (3, 3, 160, 112, 1, 5),
@@ -104,8 +118,13 @@ def test_experts_of_many_rows(counts, n, k, odd, epi):
     w = (torch.randn((len(counts), n, k), generator=gen, device="cuda") / math.sqrt(k)).bfloat16()
     offsets = torch.tensor([sum(counts[:e]) for e in range(len(counts) + 1)], dtype=torch.int32, device="cuda")
     c = torch.full((rows + 1, ldc), 7.0, dtype=torch.float32 if epi == _dense.EPI_STORE_F32 else torch.bfloat16, device="cuda")
-    _dense.check(_dense.lib().twm_dense_grouped_gemm(_dense.TWM_DENSE_BF16, a.data_ptr(), k, w.data_ptr(), k, c.data_ptr(), ldc, offsets.data_ptr(),
-                                                     len(counts), rows, n, k, epi, 0, 0, torch.cuda.current_stream().cuda_stream), "grouped_gemm")
+
+    def call():
+        _dense.check(_dense.lib().twm_dense_grouped_gemm(_dense.TWM_DENSE_BF16, a.data_ptr(), k, w.data_ptr(), k, c.data_ptr(), ldc, offsets.data_ptr(),
+                                                         len(counts), rows, n, k, epi, 0, 0, torch.cuda.current_stream().cuda_stream), "grouped_gemm")
+    names, _ = graph_nodes.captured(call)
+    assert len(names) == 1 and "gemm_experts_kernel" in names[0]
+    call()
     torch.cuda.synchronize()
     assert _dense.device_error() == 0 and bool((c[:rows, n:] == 7.0).all()) and bool((c[rows] == 7.0).all())
     want = torch.cat([a[o:o + m].double() @ w[e].double().T for e, (o, m) in enumerate(zip(offsets.tolist(), counts))])
