@@ -330,7 +330,7 @@ twm_status grouped_gemm_pairs_launch(const bf16* a, int lda, const bf16* w, int 
     g.offsets = offsets; g.experts = experts;
     if (!rows_map(&g.a_map, a, rows, K, lda, TC_BM) || !rows_map(&g.w_map, w, (long)experts * N, K, ldw, TC_BM))
         return invalid("cuTensorMapEncodeTiled refused a map of the grouped tcgen05 product");
-    return launch("gemm_tc2(grouped)", gemm_experts_kernel<EPI>, dim3(2 * (int)std::min<long>(sms / 2, (long)g.m_tiles * g.n_tiles)), TC_THREADS,
+    return launch("gemm_experts", gemm_experts_kernel<EPI>, dim3(2 * (int)std::min<long>(sms / 2, (long)g.m_tiles * g.n_tiles)), TC_THREADS,
                   Tc2Cfg<EX_TOKENS>::SMEM_BYTES, flags, stream, 2, g);
 }
 

@@ -3,9 +3,10 @@
 // The pair of CTAs and its stages are those of twm_dense_tc2.cuh with the operands' parts changed: 256 WEIGHT rows are the MMA's rows, and
 // up to 256 of an expert's activation rows its columns.  An expert's weight rows fill whole tiles; its activation rows, of any number, are
 // spread evenly over the fewest tiles and rounded up to 32, so little is multiplied for rows that are not there (128 x 256 tiles with
-// activations as rows round up to 128: an eighth more at 512 rows an expert, and the pair's 256 rows a quarter).  Bound by
-// the tensor pipe from 128 rows an expert on, by reading the weights below.  64 experts of 2048 x 1024, 512 rows each on average: 147.8 us on
-// one SM's tiles, 129.9 this way; a prompt of 4096 tokens on 16 layers of them: 11.57 -> 11.03 ms.
+// activations as rows round up to 128: an eighth more at 512 rows an expert, and the pair's 256 rows a quarter).  Below 128 rows an expert
+// bound by reading the weights.  64 experts of 2048 x 1024, 512 rows each on average: 147.8 us on one SM's tiles, 120.9 to 129.9 this way, 0.64 to
+// 0.69 of the GEMM rate: the tensor pipe is busy 67 % of the time (72 % of the time that an SM has a tile) and DRAM 47 % (every operand is read
+// once), so neither is what bounds it yet.  A prompt of 4096 tokens on 16 layers of them: 11.57 -> 11.03 ms.
 //
 // Read-back: thread = output column (its TMEM lane), 16 activation rows at a time; neighbouring threads exchange halves, so that a warp
 // stores 64 contiguous bytes of two rows.

@@ -121,9 +121,10 @@ __device__ __forceinline__ float4 scale4(const float4 x, float s, const float4 g
 // thread's share of a row is PER vectors, held in registers; PER = 0: rows
 // of any length, in shared memory.  FULL = false: without pre_norm, step, routed outputs and clear.
 //
-// Bound by latency: a row is loads, a sum over the CTA, stores.  So the factors are requested before the kernel ahead has ended, and a
+// Bound by latency: a row is loads, a sum over the CTA, stores.  So the factors, constants where kernels start early, are requested before the kernel ahead has ended, and a
 // row's loads before the row ahead of it is worked on (routed: its slots; the experts' rows are all requested at once); the host deals the rows to
-// as many CTAs as run at once.  In a prompt step, a row to a CTA (two rows' work for a shifted one) / this way: 100 rows of 2048 4.6 / 3.9 us,
+// as many CTAs as run at once (the bound on residency costs spills: 44 to 68 bytes a thread at 4 vectors a thread, 48 for routed rows of 2).  In
+// a prompt step, a row to a CTA (two rows' work for a shifted one) / this way: 100 rows of 2048 4.6 / 3.9 us,
 // 2048 rows of 3584 35.8 / 28.
 template <typename T, int PER, bool FULL>
 __global__ void __launch_bounds__(ROW_THREADS, PER == 0 || PER > 4 ? 1 : PER > 2 ? 2 : 3)

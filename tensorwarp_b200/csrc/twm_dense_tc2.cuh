@@ -2,7 +2,7 @@
 //
 // One SM's 128 x 256 tile is bound by its shared memory: 48 KB come in and go out again per 512 clocks of
 // MMA.  Here a pair of CTAs (one cluster) computes 256 x 256: each loads its own 128 activation rows and
-// HALF of the weight rows (32 KB a stage, six stages), the tensor cores of the pair share the halves
+// HALF of the weight rows (256 columns: 32 KB a stage, six stages; 224 and 192: 30 and 28 KB, seven), the tensor cores of the pair share the halves
 // (tcgen05.mma.cta_group::2, M = 256), and each CTA ends up with its 128 rows of the result in its own
 // tensor memory.  The leader's MMA thread issues for both; both CTAs' loads count on the leader's barriers;
 // a commit tells both when a stage is free and when an accumulator is complete.  A gated product takes
